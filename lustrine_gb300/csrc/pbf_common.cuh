@@ -117,6 +117,7 @@ struct SandParams {
     float attract_radius, blow_radius;
     float attract_coeff, blow_coeff;
     float radius, diameter;                 // particleRadius, particleDiameter
+    float reach2;                           // largest float whose square root rounds to at most diameter
     float w;                                // 1 / mass
 };
 
@@ -136,6 +137,28 @@ struct CellPack {
     unsigned mx, my, mz;  // per-axis masks
     int by_shift, bz_shift;
 };
+
+// Two floats in one 64-bit register pair, as a 16-byte load of a float4 leaves
+// its x, y and its z, w: sm_103a subtracts, multiplies and adds both in one
+// instruction, each half rounded to nearest as the scalar one is.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float lo2(f32x2 a) { return __uint_as_float((unsigned)a); }
+__device__ __forceinline__ float hi2(f32x2 a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
 
 __device__ __forceinline__ float dot3(float ax, float ay, float az) {
     return ax * ax + ay * ay + az * az;
@@ -183,6 +206,9 @@ bool pdl_enabled();
 // the sentinel slot n sits at SENTINEL_POS on every axis.
 constexpr int LIST_PAD_MAX = 8;
 constexpr float SENTINEL_POS = 1e18f;
+// The list builds load candidates in chunks that may reach past a cell
+// range's end: position buffers are this much longer than their particles.
+constexpr int SPAN_PAD = 8;
 
 // Cell scan of the step: tiles of CELL_TILE cells, one block each.
 constexpr int CELL_SCAN_THREADS = 256;

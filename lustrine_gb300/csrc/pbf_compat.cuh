@@ -29,4 +29,76 @@ __device__ __forceinline__ int cell_ref(const StepParams& p, float x, float y, f
     return (int)id;
 }
 
+// A thread's list entries on their way to the column rows of nbr (entry k of
+// particle i at k n + i): the first CAP wait in shared memory, entry k at
+// [k][thread], so that a candidate costs one store and a conditional step of
+// the pointer (a refused one is overwritten by the next) where a store to
+// the row under a branch would run the branch for the whole warp whenever
+// one lane accepts.  Entries past CAP (rare) go to their rows at once.
+template <int CAP, int B>
+struct StagedList {
+    int* first;  // this thread's entry 0
+    int* at;     // its next entry
+    int* row;    // nbr + i
+    size_t n;
+    int extra, max_nbrs;
+    __device__ __forceinline__ StagedList(int* smem, int* nbr, const StepParams& p, int i)
+        : first(smem + threadIdx.x), at(first), row(nbr + i), n((size_t)p.n), extra(0), max_nbrs(p.max_nbrs) {}
+    __device__ __forceinline__ bool room(int w) const { return at <= first + (CAP - w) * B; }
+    __device__ __forceinline__ void put(int e, bool in) {  // with room only
+        *at = e;
+        at += in ? B : 0;
+    }
+    __device__ __forceinline__ void push(int e) {
+        if (at < first + CAP * B) {
+            *at = e;
+            at += B;
+        } else {
+            if (CAP + extra < max_nbrs) row[(size_t)(CAP + extra) * n] = e;
+            extra++;
+        }
+    }
+    // the staged entries to their rows; the number accepted
+    __device__ __forceinline__ int close() {
+        const int m = (int)(at - first) / B;
+        for (int k = 0; k < min(m, max_nbrs); k++) row[(size_t)k * n] = first[k * B];
+        return m + extra;
+    }
+};
+
+// The particles of slots [t0, t1) of pos within h of self, in slot order,
+// entry(t) listed for each: SPAN_W positions are loaded together (past t1 too:
+// the buffers are SPAN_PAD longer), then tested in order.  The squared
+// distance is the reference's expression ((dx dx + dy dy) + dz dz, no
+// contraction), the same bits from either particle's side.
+constexpr int SPAN_W = 4;
+static_assert(SPAN_W <= SPAN_PAD, "a span reads at most SPAN_PAD positions past its end");
+template <class L, class E>
+__device__ __forceinline__ void walk_span(const float4* __restrict__ pos, int t0, int t1, const float4& self,
+                                          float h2, L& out, E&& entry) {
+    const f32x2 sxy = pack2(self.x, self.y);
+    for (int t = t0; t < t1; t += SPAN_W) {
+        const ulonglong2* __restrict__ q = reinterpret_cast<const ulonglong2*>(pos + t);
+        ulonglong2 o[SPAN_W];
+        bool in[SPAN_W];
+#pragma unroll
+        for (int u = 0; u < SPAN_W; u++) o[u] = q[u];
+        const int left = t1 - t;
+#pragma unroll
+        for (int u = 0; u < SPAN_W; u++) {
+            const f32x2 d = sub2(sxy, o[u].x), d2 = mul2(d, d);
+            const float dz = self.z - lo2(o[u].y);
+            in[u] = u < left && (lo2(d2) + hi2(d2)) + dz * dz <= h2;
+        }
+        if (out.room(SPAN_W)) {
+#pragma unroll
+            for (int u = 0; u < SPAN_W; u++) out.put(entry(t + u), in[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < SPAN_W; u++)
+                if (in[u]) out.push(entry(t + u));
+        }
+    }
+}
+
 }  // namespace lgb

@@ -277,12 +277,12 @@ static int ctx_alloc(lustrine_pbf* s) {
     int rc = LUSTRINE_OK;
     for (int k = 0; k < 2 && !rc; k++) {
         rc = rc ? rc : dalloc(&s->x[k], n);
-        rc = rc ? rc : dalloc(&s->xs[k], (size_t)n + 1);  // + the sentinel slot n
+        rc = rc ? rc : dalloc(&s->xs[k], (size_t)n + 1 + SPAN_PAD);  // + the sentinel slot n
         rc = rc ? rc : dalloc(&s->v[k], n);
         rc = rc ? rc : dalloc(&s->id[k], n);
         rc = rc ? rc : dalloc(&s->att[k], n);  // sand mode's attract flags
     }
-    rc = rc ? rc : dalloc(&s->xs_alt, (size_t)n + 1);
+    rc = rc ? rc : dalloc(&s->xs_alt, (size_t)n + 1 + SPAN_PAD);
     rc = rc ? rc : dalloc(&s->xs_pred, n);
     rc = rc ? rc : dalloc(&s->vtmp, (size_t)n + 1);
     rc = rc ? rc : dalloc(&s->key, m);
@@ -294,7 +294,7 @@ static int ctx_alloc(lustrine_pbf* s) {
     rc = rc ? rc : dalloc(&s->start, (size_t)C + 1);
     rc = rc ? rc : dalloc(&s->block_sums, scan_block_sums_size(C));
     rc = rc ? rc : dalloc(&s->tile_sum, 2 * (size_t)cell_scan_tiles(C));
-    rc = rc ? rc : dalloc(&s->solid, ns);
+    rc = rc ? rc : dalloc(&s->solid, (size_t)ns + SPAN_PAD);
     rc = rc ? rc : dalloc(&s->solid_raw, ns);
     rc = rc ? rc : dalloc(&s->sstart, (size_t)C + 1);
     const size_t list_rows = (size_t)((s->sp.max_nbrs + LIST_PAD_MAX - 1) / LIST_PAD_MAX * LIST_PAD_MAX);
@@ -706,9 +706,9 @@ static int setup_solids(lustrine_pbf* s) {
     launch_sort_tail(s->key, s->rank, s->sstart, nullptr, ns, s->tmp, s->perm, s->stream);
     launch_gather_solid(s->perm, ns, s->solid_raw, s->solid, s->stream);
     if (p.hash_bits) launch_gather_int(s->perm, ns, s->cellk, s->solid_cell, s->stream);
-    if (ns > 0) {  // PBF geometry (the reference-mode list build walks every cell)
+    if (ns > 0) {
         CK(cudaMemsetAsync(s->solid_near, 0, (size_t)C, s->stream));
-        launch_mark_solid_near(s->mixed(), p, s->cp, s->solid_raw, ns, s->solid_near, s->stream);
+        launch_mark_solid_near(s->mixed(), p, s->cp, s->solid_raw, ns, s->sstart, s->solid_near, s->stream);
     }
     CK(cudaGetLastError());
     return LUSTRINE_OK;
@@ -846,6 +846,11 @@ static SandParams sand_params(const lustrine_pbf* s) {
     q.radius = s->prm.particle_radius;
     q.diameter = c.particle_diameter;
     q.w = 1.0f / s->prm.mass;  // Simulate.cpp:185
+    // sqrt(d2) > diameter exactly when d2 > reach2 (the rounded root is monotonic)
+    q.reach2 = q.diameter * q.diameter;
+    while (std::sqrt(q.reach2) > q.diameter) q.reach2 = std::nextafter(q.reach2, 0.0f);
+    while (std::isfinite(q.reach2) && std::sqrt(std::nextafter(q.reach2, INFINITY)) <= q.diameter)
+        q.reach2 = std::nextafter(q.reach2, INFINITY);
     return q;
 }
 

@@ -323,6 +323,25 @@ __global__ void __launch_bounds__(256) k_reduce(StepParams p, CellPack cp, const
     }
 }
 
+// The marks of k_mark_solid_near on one scene's dense grid, from the sorted static particles'
+// cell table itself: a cell has one nearby when a row of its 27-cell
+// neighbourhood holds some.  Every step semantics that walks the table (each
+// bins positions with its own rounding) reads marks that agree with it.
+__global__ void k_mark_near_rows(int gx, int gy, int gz, const int* __restrict__ sstart,
+                                 unsigned char* __restrict__ near) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= gx * gy * gz) return;
+    const int z = c % gz, x = (c / gz) % gx, y = c / gz / gx;
+    const int z0 = max(z - 1, 0), z1 = min(z + 1, gz - 1);
+    bool any = false;
+    for (int yy = max(y - 1, 0); yy <= min(y + 1, gy - 1); yy++)
+        for (int xx = max(x - 1, 0); xx <= min(x + 1, gx - 1); xx++) {
+            const int row = (yy * gx + xx) * gz;
+            any |= sstart[row + z1 + 1] > sstart[row + z0];
+        }
+    near[c] = any;
+}
+
 // ------------------------------------------------------------------ launch --
 
 
@@ -344,8 +363,12 @@ void launch_predict(bool mixed, const StepParams& p, const CellPack& cp, const f
 }
 
 void launch_mark_solid_near(bool mixed, const StepParams& p, const CellPack& cp, const float4* pos, int m,
-                            unsigned char* near, cudaStream_t st) {
+                            const int* sstart, unsigned char* near, cudaStream_t st) {
     if (m <= 0) return;
+    if (!p.scenes && !p.hash_bits) {
+        k_mark_near_rows<<<blocks_for(p.num_cells, 256), 256, 0, st>>>(p.gx, p.gy, p.gz, sstart, near);
+        return;
+    }
     LGB_DISPATCH(mixed, k_mark_solid_near, blocks_for(m, 256), 256, st, p, cp, pos, m, near);
 }
 

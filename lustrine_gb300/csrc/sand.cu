@@ -95,17 +95,33 @@ __global__ void k_sand_predict(StepParams p, SandParams q, const float4* __restr
 // particle without the symmetric pushes: particle i's list is first the sand
 // particles k < i whose own walk found i, in ascending k -- the 27-cell walk
 // in y -> x -> z order visits cells by ascending id and the sorted slots of a
-// cell ascend, so that is the walk itself restricted to slots below i, with
-// the distance taken from k's side -- then its own walk over j >= i, each
-// cell's static particles before its sand.  The reference also lists i
-// itself twice; the substeps skip it (Simulate.cpp:226), so it is left out.
-// Entries: sand slot t >= 0, static slot u as -1 - u.
-__global__ void k_sand_lists(StepParams p, const float4* __restrict__ xs, const int* __restrict__ key,
-                             const int* __restrict__ fstart, const float4* __restrict__ solid,
-                             const int* __restrict__ sstart, int* __restrict__ nbr, int* __restrict__ cnt,
-                             int* status) {
+// cell ascend, so that is the walk itself restricted to slots below i -- then
+// its own walk over j >= i, each cell's static particles before its sand.
+// The reference also lists i itself twice; the substeps skip it
+// (Simulate.cpp:226), so it is left out.  Entries: sand slot t >= 0, static
+// slot u as -1 - u.
+//
+// The three cells of a row (dy, dx) are consecutive ids, so their sand is one
+// slot range.  Away from static particles (near, set per cell) the two parts
+// together are the nine ranges in order without i: one pass over the
+// candidates (two passes cell by cell took 64.6 us for 262,144 particles of a heap, h = 1.55; this
+// one takes 41.5, bound by instruction issue: 100 candidates a particle, of
+// which it lists 17).  Near some, the lower
+// slots' ranges come first, then every row's static particles with its sand
+// above i, cell by cell only in rows that hold static particles.
+constexpr int SAND_BLOCK = 128;
+// List entries staged in shared memory (16-18 a particle in a heap): at 32 the
+// larger stage leaves the L1 too small for the candidates (hit rate 80 -> 56 %,
+// 46 us), at 12 most lists leave it (49 us).
+constexpr int SAND_STAGE = 20;
+__global__ void __launch_bounds__(SAND_BLOCK) k_sand_lists(StepParams p, const float4* __restrict__ xs,
+                                                    const int* __restrict__ key, const int* __restrict__ fstart,
+                                                    const float4* __restrict__ solid,
+                                                    const int* __restrict__ sstart, int* __restrict__ nbr,
+                                                    int* __restrict__ cnt, int* status) {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ int stage[SAND_STAGE * SAND_BLOCK];
+    const int i = blockIdx.x * SAND_BLOCK + threadIdx.x;
     if (i >= p.n) return;
     const float4 self = xs[i];
     const int id = key[i];
@@ -113,45 +129,70 @@ __global__ void k_sand_lists(StepParams p, const float4* __restrict__ xs, const 
     const int yy = id / slab;
     const int t0 = id - yy * slab;
     const int zz = t0 % p.gz, xx = t0 / p.gz;
-    const int ylo = yy - 1 < 0 ? 0 : -1, yhi = yy + 1 >= p.gy ? 0 : 1;
-    const int xlo = xx - 1 < 0 ? 0 : -1, xhi = xx + 1 >= p.gx ? 0 : 1;
-    const int zlo = zz - 1 < 0 ? 0 : -1, zhi = zz + 1 >= p.gz ? 0 : 1;
-    int c_n = 0;
-    // sand below i that found i: cells up to its own (later cells hold later slots)
-    for (int y = ylo; y <= 0; y++)
-        for (int x = (y < 0 ? xlo : max(xlo, -1)); x <= (y < 0 ? xhi : 0); x++)
-            for (int z = zlo; z <= ((y < 0 || x < 0) ? zhi : 0); z++) {
-                const int c = (yy + y) * slab + (xx + x) * p.gz + (zz + z);
-                const int e = min(fstart[c + 1], i);
-                for (int t = fstart[c]; t < e; t++) {
-                    const float4 o = xs[t];
-                    if (sdot(o.x - self.x, o.y - self.y, o.z - self.z) <= p.h2) {
-                        if (c_n < p.max_nbrs) nbr[(size_t)c_n * p.n + i] = t;
-                        c_n++;
-                    }
+    const int z0 = max(zz - 1, 0), z1 = min(zz + 1, p.gz - 1);
+    const bool near = p.ns > 0 && p.solid_near[id];
+    StagedList<SAND_STAGE, SAND_BLOCK> out(stage, nbr, p, i);
+    auto sand_entry = [](int t) { return t; };
+    auto static_entry = [](int u) { return -1 - u; };
+    // the ranges: i's own row is cut at i into two, and near static particles
+    // only those up to i come here; each range's bounds are loaded while the
+    // one before is walked
+    const int spans = near ? 5 : 10;
+    int next = 0, a_next = 0, b_next = 0, s_next = 0, e_next = 0;
+    auto bounds = [&](int r) {
+        for (; r < spans; r++) {
+            const int k = r > 4 ? r - 1 : r;
+            const int y = yy + k / 3 - 1, x = xx + k % 3 - 1;
+            if (y < 0 || y >= p.gy || x < 0 || x >= p.gx) continue;
+            const int row = y * slab + x * p.gz;
+            a_next = r == 5 ? i + 1 : fstart[row + z0];
+            b_next = r == 4 ? i : fstart[row + z1 + 1];
+            break;
+        }
+        next = r;
+    };
+    bounds(0);
+    while (next < spans) {
+        const int a = a_next, b = b_next;
+        bounds(next + 1);
+        walk_span(xs, a, b, self, p.h2, out, sand_entry);
+    }
+    if (near) {
+        auto rows = [&](int r) {  // the next row from r on: its static particles, and its sand above i
+            for (; r < 9; r++) {
+                const int y = yy + r / 3 - 1, x = xx + r % 3 - 1;
+                if (y < 0 || y >= p.gy || x < 0 || x >= p.gx) continue;
+                const int row = y * slab + x * p.gz;
+                s_next = sstart[row + z0];
+                e_next = sstart[row + z1 + 1];
+                a_next = r < 4 ? 0 : (r == 4 ? i + 1 : fstart[row + z0]);
+                b_next = r < 4 ? 0 : fstart[row + z1 + 1];
+                if (s_next < e_next || a_next < b_next) break;
+            }
+            next = r;
+        };
+        rows(0);
+        while (next < 9) {
+            const int r = next, a = a_next, b = b_next, sa = s_next, sb = e_next;
+            rows(r + 1);
+            if (a >= b) {
+                walk_span(solid, sa, sb, self, p.h2, out, static_entry);
+            } else if (sa == sb) {
+                walk_span(xs, a, b, self, p.h2, out, sand_entry);
+            } else {
+                const int row = (yy + r / 3 - 1) * slab + (xx + r % 3 - 1) * p.gz;
+                int s0 = sa, f0 = a;  // both advance cell by cell
+                for (int c = row + z0; c <= row + z1; c++) {
+                    const int s1 = sstart[c + 1], f1 = fstart[c + 1];
+                    walk_span(solid, s0, s1, self, p.h2, out, static_entry);
+                    walk_span(xs, f0, f1, self, p.h2, out, sand_entry);
+                    s0 = s1;
+                    f0 = max(f0, f1);
                 }
             }
-    // its own walk: static particles, then sand above i (cells from its own on)
-    for (int y = ylo; y <= yhi; y++)
-        for (int x = xlo; x <= xhi; x++)
-            for (int z = zlo; z <= zhi; z++) {
-                const int c = (yy + y) * slab + (xx + x) * p.gz + (zz + z);
-                for (int u = sstart[c], e = sstart[c + 1]; u < e; u++) {
-                    const float4 o = solid[u];
-                    if (sdot(self.x - o.x, self.y - o.y, self.z - o.z) <= p.h2) {
-                        if (c_n < p.max_nbrs) nbr[(size_t)c_n * p.n + i] = -1 - u;
-                        c_n++;
-                    }
-                }
-                if (c < id) continue;
-                for (int t = max(fstart[c], i + 1), e = fstart[c + 1]; t < e; t++) {
-                    const float4 o = xs[t];
-                    if (sdot(self.x - o.x, self.y - o.y, self.z - o.z) <= p.h2) {
-                        if (c_n < p.max_nbrs) nbr[(size_t)c_n * p.n + i] = t;
-                        c_n++;
-                    }
-                }
-            }
+        }
+    }
+    int c_n = out.close();
     if (c_n > p.max_nbrs) {
         set_status(status, ST_NBR_OVERFLOW);
         c_n = p.max_nbrs;
@@ -160,43 +201,34 @@ __global__ void k_sand_lists(StepParams p, const float4* __restrict__ xs, const 
 }
 
 // One contact and friction term (Simulate.cpp:236-266 for a sand neighbour,
-// 268-286 for a static one), subtracted from dp.
-template <bool SAND_J>
-__device__ __forceinline__ void sand_pair(const StepParams& p, const SandParams& q, float4 pi, float4 pj,
+// 268-286 for a static one), subtracted from dp.  coef: the contact's share,
+// collision m / (m + m) between two sand particles, collision against a
+// static one (whose own displacement is zero).
+__device__ __forceinline__ void sand_pair(const SandParams& q, bool sand_j, float coef, float4 pi, float4 pj,
                                           float4 xi, float4 xj, float& dpx, float& dpy, float& dpz) {
     float ix = pi.x - pj.x, iy = pi.y - pj.y, iz = pi.z - pj.z;
-    if (slen(ix, iy, iz) == 0.0f) {
+    float d2 = sdot(ix, iy, iz);
+    if (d2 == 0.0f) {
         ix = 0.0f;
         iy = 0.00001f;
         iz = 0.0f;
+        d2 = sdot(ix, iy, iz);
     }
-    const float len = slen(ix, iy, iz);
+    const float len = sqrtf(d2);
     if (len > q.diameter) return;
-    const float s = SAND_J ? ((SAND_COLLISION * p.mass) / (p.mass + p.mass)) * (len - q.diameter)
-                           : SAND_COLLISION * (len - q.diameter);
+    const float s = coef * (len - q.diameter);
     const float tx = (s * ix) / len, ty = (s * iy) / len, tz = (s * iz) / len;
     dpx = dpx - tx;
     dpy = dpy - ty;
     dpz = dpz - tz;
     const float d = slen(tx, ty, tz);
     const float ax = pi.x - tx, ay = pi.y - ty, az = pi.z - tz;  // pi - tmp
-    float rx, ry, rz, nx, ny, nz;
-    if (SAND_J) {
-        const float bx = pj.x + tx, by = pj.y + ty, bz = pj.z + tz;  // pj + tmp
-        rx = (ax - xi.x) - (bx - xj.x);
-        ry = (ay - xi.y) - (by - xj.y);
-        rz = (az - xi.z) - (bz - xj.z);
-        nx = ax - bx;
-        ny = ay - by;
-        nz = az - bz;
-    } else {
-        rx = (ax - xi.x) - 0.0f;
-        ry = (ay - xi.y) - 0.0f;
-        rz = (az - xi.z) - 0.0f;
-        nx = ax - pj.x;
-        ny = ay - pj.y;
-        nz = az - pj.z;
-    }
+    // pj + tmp and its displacement; a static particle stays
+    const float bx = sand_j ? pj.x + tx : pj.x, by = sand_j ? pj.y + ty : pj.y, bz = sand_j ? pj.z + tz : pj.z;
+    const float rx = (ax - xi.x) - (sand_j ? bx - xj.x : 0.0f);
+    const float ry = (ay - xi.y) - (sand_j ? by - xj.y : 0.0f);
+    const float rz = (az - xi.z) - (sand_j ? bz - xj.z : 0.0f);
+    float nx = ax - bx, ny = ay - by, nz = az - bz;
     const float inv = 1.0f / sqrtf(sdot(nx, ny, nz));
     nx = nx * inv;
     ny = ny * inv;
@@ -224,25 +256,62 @@ __device__ __forceinline__ void sand_pair(const StepParams& p, const SandParams&
 // particle's index -- its slot in this step's cell order, as the reference
 // re-orders its arrays -- into the side the step started from (whose
 // contents the sort already consumed).
-__global__ void k_sand_substep(StepParams p, SandParams q, const float4* __restrict__ tmp_in,
-                               float4* __restrict__ star_out, const float4* __restrict__ xpre,
-                               const int* __restrict__ nbr, const int* __restrict__ cnt,
-                               const float4* __restrict__ solid, float4* __restrict__ x_commit,
-                               float4* __restrict__ v_commit, const int* __restrict__ att_in,
-                               int* __restrict__ att_commit, int* __restrict__ id_commit) {
+//
+// A list holds every particle within h, a third of them in contact (within a
+// diameter), and a contact term costs some 150 instructions (four square
+// roots and five divisions, each correctly rounded).  Evaluated entry by entry a
+// warp pays for a term wherever any lane has a contact (13 of 32 lanes active).
+// So a thread first collects its contacts: SAND_CHUNK positions loaded
+// together (2 or 8: 10 % slower) and tested by d^2 against reach2, the largest
+// float whose square root rounds to at most the diameter (the same test
+// without the root); then it evaluates them in list order, the next contact's
+// positions loaded ahead.
+constexpr int SAND_CHUNK = 4;
+constexpr int SAND_HITS = 16;  // contacts collected before they are evaluated
+__global__ void __launch_bounds__(SAND_BLOCK) k_sand_substep(
+    StepParams p, SandParams q, const float4* __restrict__ tmp_in, float4* __restrict__ star_out,
+    const float4* __restrict__ xpre, const int* __restrict__ nbr, const int* __restrict__ cnt,
+    const float4* __restrict__ solid, float4* __restrict__ x_commit, float4* __restrict__ v_commit,
+    const int* __restrict__ att_in, int* __restrict__ att_commit, int* __restrict__ id_commit) {
     pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ int hits[SAND_HITS * SAND_BLOCK];
+    const int i = blockIdx.x * SAND_BLOCK + threadIdx.x;
     if (i >= p.n) return;
+    int* hit = hits + threadIdx.x;
     const float4 pi = tmp_in[i];
     const float4 xi = xpre[i];
+    const float sand_coef = (SAND_COLLISION * p.mass) / (p.mass + p.mass);
     float dpx = 0.0f, dpy = 0.0f, dpz = 0.0f;
     const int c = cnt[i];
-    for (int k = 0; k < c; k++) {
-        const int e = nbr[(size_t)k * p.n + i];
-        if (e >= 0)
-            sand_pair<true>(p, q, pi, tmp_in[e], xi, xpre[e], dpx, dpy, dpz);
-        else
-            sand_pair<false>(p, q, pi, __ldg(&solid[-1 - e]), xi, xi, dpx, dpy, dpz);
+    auto pos = [&](int e) { return e >= 0 ? tmp_in[e] : __ldg(&solid[-1 - e]); };
+    for (int k = 0; k < c;) {
+        int m = 0;
+        for (; k < c && m <= SAND_HITS - SAND_CHUNK; k += SAND_CHUNK) {
+            int e[SAND_CHUNK];
+            float4 o[SAND_CHUNK];
+#pragma unroll
+            for (int u = 0; u < SAND_CHUNK; u++) e[u] = nbr[(size_t)min(k + u, c - 1) * p.n + i];
+#pragma unroll
+            for (int u = 0; u < SAND_CHUNK; u++) o[u] = pos(e[u]);
+#pragma unroll
+            for (int u = 0; u < SAND_CHUNK; u++) {
+                const float d2 = sdot(pi.x - o[u].x, pi.y - o[u].y, pi.z - o[u].z);
+                if (k + u < c && !(d2 > q.reach2)) hit[SAND_BLOCK * m++] = e[u];
+            }
+        }
+        if (!m) continue;
+        int e = hit[0];
+        float4 pj = pos(e), xj = e >= 0 ? xpre[e] : pj;
+        for (int h = 0; h < m; h++) {
+            const bool sand_j = e >= 0;
+            const float4 pc = pj, xc = xj;
+            if (h + 1 < m) {
+                e = hit[SAND_BLOCK * (h + 1)];
+                pj = pos(e);
+                xj = e >= 0 ? xpre[e] : pj;
+            }
+            sand_pair(q, sand_j, sand_j ? sand_coef : SAND_COLLISION, pi, pc, xi, xc, dpx, dpy, dpz);
+        }
     }
     const float4 s = sand_clamp(p, pi.x + dpx, pi.y + dpy, pi.z + dpz);
     if (!x_commit) {
@@ -270,7 +339,7 @@ void launch_sand_lists(const StepParams& p, const float4* xs, const int* key, co
                        const float4* solid, const int* sstart, int* nbr, int* cnt, int* status,
                        cudaStream_t st) {
     if (p.n <= 0) return;
-    launch_k(k_sand_lists, blocks_for(p.n, 128), 128, st, pdl_enabled(), p, xs, key, fstart, solid, sstart,
+    launch_k(k_sand_lists, blocks_for(p.n, SAND_BLOCK), SAND_BLOCK, st, pdl_enabled(), p, xs, key, fstart, solid, sstart,
              nbr, cnt, status);
 }
 
@@ -279,8 +348,8 @@ void launch_sand_substep(const StepParams& p, const SandParams& q, const float4*
                          float4* x_commit, float4* v_commit, const int* att_in, int* att_commit,
                          int* id_commit, cudaStream_t st) {
     if (p.n <= 0) return;
-    launch_k(k_sand_substep, blocks_for(p.n, 128), 128, st, pdl_enabled(), p, q, tmp_in, star_out, xpre, nbr,
-             cnt, solid, x_commit, v_commit, att_in, att_commit, id_commit);
+    launch_k(k_sand_substep, blocks_for(p.n, SAND_BLOCK), SAND_BLOCK, st, pdl_enabled(), p, q, tmp_in, star_out,
+             xpre, nbr, cnt, solid, x_commit, v_commit, att_in, att_commit, id_commit);
 }
 
 }  // namespace lgb
