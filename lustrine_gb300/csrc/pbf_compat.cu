@@ -15,9 +15,28 @@
 
 namespace lgb {
 
+// a / b correctly rounded from y = 1 / b correctly rounded, the divisor known
+// in advance (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Comput. 2004): a product, its remainder, one correction, where a division
+// that knows neither takes some 13 instructions.  The remainder has to be
+// exact: a not below 2^-100 or zero (its sign kept), b within 2^-60 .. 2^60.
+__device__ __forceinline__ float div_known(float a, float b, float y) {
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(-__fmaf_rn(b, q, -a), y, q);
+}
+
+// q = r kfac / h of the kernels.  rcp_h: 1 / h, or 0 where h is out of
+// div_known's range.  (Below 2^-100 the quotient's last bits may differ: W is
+// then its value at 0 and the gradient 0 either way.)
+__device__ __forceinline__ float q_ref(const StepParams& p, float r) {
+    const float rl = r * p.kfac;
+    return p.rcp_h != 0.0f ? div_known(rl, p.h, p.rcp_h) : rl / p.h;
+}
+
 // cubic_kernel (Kernels.cpp:6-19)
 __device__ __forceinline__ float W_ref(const StepParams& p, float r) {
-    float q = (r * p.kfac) / p.h;
+    float q = q_ref(p, r);
     float result = 0.0f;
     if (q <= 1.0f) {
         if (q <= 0.5f) {
@@ -37,9 +56,11 @@ __device__ __forceinline__ float W_ref(const StepParams& p, float r) {
 // callers already hold (the same expression, so the same bits)
 __device__ __forceinline__ float3 gradW_ref(const StepParams& p, float rx, float ry, float rz, float len) {
     float rl = len * p.kfac;
-    float q = rl / p.h;
+    float q = q_ref(p, len);
     float3 out = make_float3(0.0f, 0.0f, 0.0f);
-    if ((double)rl > 1.0e-5 && q <= 1.0f) {
+    // the reference compares with the double 1.0e-5, which lies between the
+    // float 1.0e-5f and the next: the same comparison
+    if (rl > 1.0e-5f && q <= 1.0f) {
         float s = 1.0f / (rl * p.h);
         float gx = s * rx, gy = s * ry, gz = s * rz;
         float c;
@@ -54,10 +75,13 @@ __device__ __forceinline__ float3 gradW_ref(const StepParams& p, float rx, float
     return out;
 }
 
-// s_coor (Simulate.cpp:7-9): -k * pow(W(r) / W(dq), n)
-__device__ __forceinline__ float scorr_ref(const StepParams& p, float rl, float w_dq) {
-    float ratio = W_ref(p, rl) / w_dq;
-    float pw = p.sn_int >= 0 ? ipow_rn(ratio, p.sn_int) : powf(ratio, p.sn);
+// s_coor (Simulate.cpp:7-9): -k * pow(W(r) / W(dq), n).  rcp_w: 1 / W(dq) at
+// the exponent 4, or 0 where W(dq) is out of div_known's range (a W(r) below
+// it gives a power that underflows to 0 either way).
+__device__ __forceinline__ float scorr_ref(const StepParams& p, float rl, float w_dq, float rcp_w) {
+    const float w = W_ref(p, rl);
+    float ratio = rcp_w != 0.0f ? div_known(w, w_dq, rcp_w) : w / w_dq;
+    float pw = p.sn_int == 4 ? pow4_rn(ratio) : (p.sn_int >= 0 ? ipow_rn(ratio, p.sn_int) : powf(ratio, p.sn));
     return (-p.sk) * pw;
 }
 
@@ -103,55 +127,70 @@ __global__ void k_key_ref(StepParams p, const float4* __restrict__ pos, int m, i
 // Neighbours in the reference's list order: the 27 cells around the
 // particle's cell in y -> x -> z offset order (Neighbors.cpp:401-403); in each
 // cell its fluid particles by ascending id, then its solids by ascending
-// storage index (Neighbors.cpp:374-384).
-__global__ void k_lists_ref(StepParams p, const float4* __restrict__ xs, const int* __restrict__ key,
-                            const int* __restrict__ fstart, const float4* __restrict__ solid,
-                            const int* __restrict__ sstart, int* __restrict__ nbr,
-                            int* __restrict__ cnt, int* status) {
+// storage index (Neighbors.cpp:374-384).  The three cells of a row are
+// consecutive ids: a row without solids is one range of fluid slots, walked
+// in one loop; the solids' table is read only near solids (near, set per
+// cell).  Each row's bounds are loaded while the one before is walked.  Bound by
+// instruction issue at the few warps a scene of this mode has (100,000
+// particles, h = 1.55: 36.2 us cell by cell with a store to the list's row per
+// accepted candidate, 19.5 us like this).
+constexpr int REF_BLOCK = 128;
+constexpr int REF_STAGE = 24;  // list entries staged in shared memory
+__global__ void __launch_bounds__(REF_BLOCK) k_lists_ref(StepParams p, const float4* __restrict__ xs,
+                                                         const int* __restrict__ key,
+                                                         const int* __restrict__ fstart,
+                                                         const float4* __restrict__ solid,
+                                                         const int* __restrict__ sstart, int* __restrict__ nbr,
+                                                         int* __restrict__ cnt, int* status) {
     pdl_wait();
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ int stage[REF_STAGE * REF_BLOCK];
+    const int s = blockIdx.x * REF_BLOCK + threadIdx.x;
     if (s >= p.n) return;
     const float4 self = xs[s];
     const int id = key[s];
     const int slab = p.gx * p.gz;
     const int yy = id / slab, xx = (id % slab) / p.gz, zz = id % p.gz;
-    int c_n = 0;
-    // a row's cells z-1 .. z+1 are consecutive ids: their fluid and solid
-    // ranges come from four loads of each table; the cells are still walked
-    // one by one, fluid before solids, as the reference lists them
     const int z0 = max(zz - 1, 0), z1 = min(zz + 1, p.gz - 1);
-    for (int y = -1; y <= 1; y++)
-        for (int x = -1; x <= 1; x++) {
-            if (xx + x < 0 || xx + x >= p.gx || yy + y < 0 || yy + y >= p.gy) continue;
-            const int row = (yy + y) * slab + (xx + x) * p.gz;
-            int fb[4], sb[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const bool in = z0 + k <= z1 + 1;
-                fb[k] = in ? __ldg(&fstart[row + z0 + k]) : 0;
-                sb[k] = in ? __ldg(&sstart[row + z0 + k]) : 0;
+    const bool near = p.ns > 0 && p.solid_near[id];
+    StagedList<REF_STAGE, REF_BLOCK> out(stage, nbr, p, s);
+    auto fluid_entry = [](int t) { return t; };
+    auto solid_entry = [](int u) { return -1 - u; };
+    int next = 0, row = 0, a_next = 0, b_next = 0, s_next = 0, e_next = 0;
+    auto bounds = [&](int r) {
+        for (; r < 9; r++) {
+            const int y = yy + r / 3 - 1, x = xx + r % 3 - 1;
+            if (y < 0 || y >= p.gy || x < 0 || x >= p.gx) continue;
+            row = y * slab + x * p.gz;
+            a_next = fstart[row + z0];
+            b_next = fstart[row + z1 + 1];
+            if (near) {
+                s_next = sstart[row + z0];
+                e_next = sstart[row + z1 + 1];
             }
-#pragma unroll
-            for (int k = 0; k < 3; k++) {
-                if (z0 + k > z1) break;
-                for (int t = fb[k]; t < fb[k + 1]; t++) {
-                    float4 o = xs[t];
-                    float dx = self.x - o.x, dy = self.y - o.y, dz = self.z - o.z;
-                    if ((dx * dx + dy * dy) + dz * dz <= p.h2) {
-                        if (c_n < p.max_nbrs) nbr[(size_t)c_n * p.n + s] = t;
-                        c_n++;
-                    }
-                }
-                for (int t = sb[k]; t < sb[k + 1]; t++) {
-                    float4 o = __ldg(&solid[t]);
-                    float dx = self.x - o.x, dy = self.y - o.y, dz = self.z - o.z;
-                    if ((dx * dx + dy * dy) + dz * dz <= p.h2) {
-                        if (c_n < p.max_nbrs) nbr[(size_t)c_n * p.n + s] = -1 - t;
-                        c_n++;
-                    }
-                }
+            break;
+        }
+        next = r;
+    };
+    bounds(0);
+    while (next < 9) {
+        const int a = a_next, b = b_next, sa = s_next, sb = e_next, r0 = row;
+        bounds(next + 1);
+        if (sa == sb) {
+            walk_span(xs, a, b, self, p.h2, out, fluid_entry);
+        } else if (a == b) {
+            walk_span(solid, sa, sb, self, p.h2, out, solid_entry);
+        } else {
+            int f0 = a, s0 = sa;
+            for (int c = r0 + z0; c <= r0 + z1; c++) {
+                const int f1 = fstart[c + 1], s1 = sstart[c + 1];
+                walk_span(xs, f0, f1, self, p.h2, out, fluid_entry);
+                walk_span(solid, s0, s1, self, p.h2, out, solid_entry);
+                f0 = f1;
+                s0 = s1;
             }
         }
+    }
+    int c_n = out.close();
     if (c_n > p.max_nbrs) {
         set_status(status, ST_NBR_OVERFLOW);
         c_n = p.max_nbrs;
@@ -162,6 +201,28 @@ __global__ void k_lists_ref(StepParams p, const float4* __restrict__ xs, const i
 __device__ __forceinline__ float4 nbr_pos(int j, const float4* __restrict__ xs,
                                           const float4* __restrict__ solid) {
     return j >= 0 ? xs[j] : solid[-1 - j];
+}
+
+// f(k, position) for every entry k of a list, in order: REF_CHUNK entries and
+// then their positions are loaded together, the next chunk's entries while
+// this one is used (2 or 8: no faster).
+constexpr int REF_CHUNK = 4;
+template <class F>
+__device__ __forceinline__ void for_each_nbr(const StepParams& p, const int* __restrict__ nbr, int s, int c,
+                                             const float4* __restrict__ xs, const float4* __restrict__ solid, F&& f) {
+    int e[REF_CHUNK];
+#pragma unroll
+    for (int u = 0; u < REF_CHUNK; u++) e[u] = c > 0 ? __ldg(&nbr[(size_t)min(u, c - 1) * p.n + s]) : 0;
+    for (int k = 0; k < c; k += REF_CHUNK) {
+        float4 o[REF_CHUNK];
+#pragma unroll
+        for (int u = 0; u < REF_CHUNK; u++) o[u] = nbr_pos(e[u], xs, solid);
+#pragma unroll
+        for (int u = 0; u < REF_CHUNK; u++) e[u] = __ldg(&nbr[(size_t)min(k + REF_CHUNK + u, c - 1) * p.n + s]);
+#pragma unroll
+        for (int u = 0; u < REF_CHUNK; u++)
+            if (k + u < c) f(k + u, o[u]);
+    }
 }
 
 // Simulate.cpp:58-88; lambdas are stored by the caller's particle id because
@@ -182,11 +243,7 @@ __global__ void k_lambda_ref(StepParams p, const float4* __restrict__ xs, const 
     float gsum = 0.0f;
     float gcx = 0.0f, gcy = 0.0f, gcz = 0.0f;
     const float coef = -(p.mass / p.rho0);
-    int e_next = c > 0 ? __ldg(&nbr[s]) : 0;
-    for (int k = 0; k < c; k++) {
-        const int e = e_next;
-        if (k + 1 < c) e_next = __ldg(&nbr[(size_t)(k + 1) * p.n + s]);  // next entry while this one is used
-        float4 o = nbr_pos(e, xs, solid);
+    for_each_nbr(p, nbr, s, c, xs, solid, [&](int, float4 o) {
         float ix = self.x - o.x, iy = self.y - o.y, iz = self.z - o.z;
         float len = sqrtf((ix * ix + iy * iy) + iz * iz);
         density += p.mass * W_ref(p, len);
@@ -196,9 +253,9 @@ __global__ void k_lambda_ref(StepParams p, const float4* __restrict__ xs, const 
         gcx -= nx;
         gcy -= ny;
         gcz -= nz;
-    }
+    });
     density += p.mass * W_ref(p, 0.0f);
-    float constraint = (float)((double)(density / p.rho0) - 1.0);
+    float constraint = density / p.rho0 - 1.0f;  // exact in the reference's double, then rounded: the same value
     gsum += (gcx * gcx + gcy * gcy) + gcz * gcz;
     float lam = 0.0f;
     if (gsum > 0.0f) lam = (-constraint) / (gsum + p.eps);
@@ -206,7 +263,9 @@ __global__ void k_lambda_ref(StepParams p, const float4* __restrict__ xs, const 
     if (rho) rho[s] = density;
 }
 
-// Simulate.cpp:90-113 with a Jacobi read of the neighbours' positions.
+// Simulate.cpp:90-113 with a Jacobi read of the neighbours' positions.  Bound
+// by instruction issue; s_corr's power in double and the two divisions took
+// more than half of it (100,000 particles of 27 neighbours: 47.4 us, now 20.6).
 __global__ void k_delta_ref(StepParams p, const float4* __restrict__ xs, float4* __restrict__ xs_out,
                             float4* __restrict__ x, float4* __restrict__ v,
                             const int* __restrict__ id, const int* __restrict__ nbr,
@@ -218,22 +277,19 @@ __global__ void k_delta_ref(StepParams p, const float4* __restrict__ xs, float4*
     const float4 self = xs[s];
     const float li = lam_by_id[id[s]];
     const float w_dq = W_ref(p, p.dq);
+    const float rcp_w = p.sn_int == 4 && w_dq >= 0x1p-40f && w_dq <= 0x1p60f ? __frcp_rn(w_dq) : 0.0f;
     const int c = cnt[s];
     float px = 0.0f, py = 0.0f, pz = 0.0f;
-    int e_next = c > 0 ? __ldg(&nbr[s]) : 0;
-    for (int k = 0; k < c; k++) {
-        const int e = e_next;
-        if (k + 1 < c) e_next = __ldg(&nbr[(size_t)(k + 1) * p.n + s]);
-        float4 o = nbr_pos(e, xs, solid);
+    for_each_nbr(p, nbr, s, c, xs, solid, [&](int k, float4 o) {
         float ix = self.x - o.x, iy = self.y - o.y, iz = self.z - o.z;
         float len = sqrtf((ix * ix + iy * iy) + iz * iz);
-        float sc = scorr_ref(p, len, w_dq);
+        float sc = scorr_ref(p, len, w_dq, rcp_w);
         float3 g = gradW_ref(p, ix, iy, iz, len);
         float w = (li + lam_by_id[k]) + sc;
         px += w * g.x;
         py += w * g.y;
         pz += w * g.z;
-    }
+    });
     px = px / p.rho0;
     py = py / p.rho0;
     pz = pz / p.rho0;
@@ -268,7 +324,7 @@ void launch_lists_ref(const StepParams& p, const float4* xs, const int* key, con
                       const float4* solid, const int* sstart, int* nbr, int* cnt, int* status,
                       cudaStream_t st) {
     if (p.n <= 0) return;
-    launch_k(k_lists_ref, blocks_for(p.n, 128), 128, st, pdl_enabled(), p, xs, key, fstart, solid, sstart, nbr,
+    launch_k(k_lists_ref, blocks_for(p.n, REF_BLOCK), REF_BLOCK, st, pdl_enabled(), p, xs, key, fstart, solid, sstart, nbr,
              cnt, status);
 }
 

@@ -125,6 +125,7 @@ static int derive(const lustrine_pbf_params& q, int n, int ns, StepParams* sp, C
     p.h = q.kernel_radius;
     p.h2 = q.kernel_radius * q.kernel_radius;
     p.kfac = q.kernel_factor;
+    p.rcp_h = (p.h >= 0x1p-30f && p.h <= 0x1p30f) ? 1.0f / p.h : 0.0f;
     {
         float h3 = (float)std::pow((double)q.kernel_radius, 3);
         p.cubic_k = (float)(8.0 / (kPi * (double)h3));
