@@ -519,11 +519,15 @@ LUSTRINE_API int lustrine_pbf_launches_per_step(const lustrine_pbf* s);
  * input index of the k-th smallest key (equal keys in input order) and
  * counts (num_cells + 1 ints) the state the reference leaves in its counts
  * array: the first output position of every key, then num_positions.  The
- * extra scratch is taken with cudaMallocAsync on `stream` (a cudaStream_t,
- * NULL for the default stream) and returned before the call ends; the call
- * synchronises the stream.  LUSTRINE_ERR_ARGS if a key is out of range. */
+ * extra scratch is taken from a pool of the library's own in the order of
+ * `stream` (a cudaStream_t, NULL for the default stream) and returned to it
+ * before the call ends; the call synchronises the stream.  The pool keeps up to
+ * 128 MiB a device for later calls.  LUSTRINE_ERR_ARGS if a key is out of range. */
 LUSTRINE_API int lustrine_counting_sort(int* counts, const int* keys, size_t num_positions,
                                         size_t num_cells, int* sorted_indices, void* stream);
+/* Gives the scratch that lustrine_counting_sort keeps on the current device
+ * back to the system (a later call takes it anew). */
+LUSTRINE_API int lustrine_release_scratch(void);
 
 /* No counterpart in the reference.  The same sort for callers that cannot
  * allocate GPU memory while they run (an engine that budgets all device

@@ -704,7 +704,7 @@ static int setup_solids(lustrine_pbf* s) {
                        s->stream);
     }
     launch_scan(s->count, C, s->block_sums, s->sstart, s->stream);
-    launch_sort_tail(s->key, s->rank, s->sstart, nullptr, ns, s->tmp, s->perm, s->stream);
+    launch_sort_tail(s->key, C, s->rank, s->sstart, nullptr, ns, s->tmp, s->perm, s->stream);
     launch_gather_solid(s->perm, ns, s->solid_raw, s->solid, s->stream);
     if (p.hash_bits) launch_gather_int(s->perm, ns, s->cellk, s->solid_cell, s->stream);
     if (ns > 0) {

@@ -14,10 +14,10 @@ constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr size_t scan_block_sums_ints(size_t C) { return (C + SCAN_TILE - 1) / SCAN_TILE + 1; }
-// Scratch of the standalone counting sort: count[C], the scan's tile sums,
-// key[n], rank[n] (also the big cells' merge space), tmp[n], status.
+// Scratch of the standalone counting sort: count[C], status, the scan's tile
+// sums, rank[n] (also the big cells' merge space), tmp[n].
 constexpr size_t counting_sort_scratch_ints_for(size_t n, size_t C) {
-    return C + scan_block_sums_ints(C) + 3 * n + 1;
+    return C + 1 + scan_block_sums_ints(C) + 2 * n;
 }
 // exclusive scan count -> start (C + 1 entries); zeroes count behind it
 void launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st);
@@ -33,22 +33,21 @@ void launch_scan_tiles(int* count, int C, int* tile_sum, int* start, cudaStream_
                        int* tile_zero = nullptr);
 int scan_tiles_launches(int C, bool counted = false);
 // rank doubles as merge space for cells of more than a few dozen particles
-void launch_sort_tail(const int* key, int* rank, const int* start, const int* tie, int n,
+void launch_sort_tail(const int* key, int num_cells, int* rank, const int* start, const int* tie, int n,
                       int* tmp, int* perm, cudaStream_t st);
 void launch_gather_state(const int* perm, int n, const int* key, const float4* x, const float4* xs,
                          const float4* v, const int* id, int* key_out, float4* x_out,
                          float4* xs_out, float4* v_out, int* id_out, cudaStream_t st);
 void launch_gather_solid(const int* perm, int n, const float4* src, float4* dst, cudaStream_t st);
 // Standalone stable counting sort of caller keys (Sorting::counting_sort,
-// src/neighbors/Sorting.cpp:12-34): scratch carved from one int buffer whose
-// count part must be zero on entry (the scan leaves it zero again).
+// src/neighbors/Sorting.cpp:12-34): scratch carved from one 16-byte aligned int
+// buffer whose count and status must be zero on entry.
 struct CountingSortScratch {
     int* count;       // num_cells
-    int* block_sums;  // scan_block_sums_size(num_cells)
-    int* key;         // n (validated keys)
+    int* status;      // 1: set to ST_BAD_VALUE by a key out of range
+    int* block_sums;  // scan_block_sums_size(num_cells), or the step scan's tile totals
     int* rank;        // n
     int* tmp;         // n
-    int* status;      // 1
 };
 size_t counting_sort_scratch_ints(int n, int num_cells);
 CountingSortScratch counting_sort_scratch(int* base, int n, int num_cells);

@@ -31,8 +31,8 @@ using namespace lgb;
 
 namespace {
 
-// the sort's scratch (count[cells] + scan tile sums + key, rank, tmp[keys] +
-// status) at the maxima, sized by the same layout function the sort uses
+// the sort's scratch (count[cells] + status + scan tile sums + rank, tmp[keys])
+// at the maxima, sized by the same layout function the sort uses
 constexpr size_t kScratchInts =
     counting_sort_scratch_ints_for((size_t)LUSTRINE_NOALLOC_MAX_KEYS, (size_t)LUSTRINE_NOALLOC_MAX_CELLS);
 static_assert(kScratchInts * sizeof(int) <= LUSTRINE_NOALLOC_SCRATCH_BYTES,
@@ -80,8 +80,7 @@ extern "C" int lustrine_counting_sort_noalloc(int* counts, const int* keys, size
     CountingSortScratch w = counting_sort_scratch(scratch, n, C);
     // the histogram and the status word start at zero; the rest is written
     // before it is read
-    cudaError_t e = cudaMemsetAsync(w.count, 0, (size_t)C * sizeof(int), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(w.status, 0, sizeof(int), st);
+    cudaError_t e = cudaMemsetAsync(w.count, 0, ((size_t)C + 1) * sizeof(int), st);
     if (e != cudaSuccess) return lgb_cuda_status(e, "cudaMemsetAsync");
     launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
     int bad = 0;
