@@ -260,14 +260,12 @@ __device__ __forceinline__ int cell_key(const StepParams& p, const CellPack& cp,
 // fused multiply-adds keep the arithmetic identical wherever it is inlined:
 // the prediction kernel and the commit kernel of the previous step (which
 // predicts the next step when nothing changes in between) agree bit for bit.
-// tile_count (may be null): the cell scan's per-tile totals, counted here
-// with one atomic per tile a warp's particles fall in (slots are in cell
-// order, so a warp's keys share a tile of CELL_TILE cells nearly always).
+// Returns the cell key.
 template <bool MIXED>
-__device__ __forceinline__ void predict_one(const StepParams& p, const CellPack& cp, const Geo& g, float4 xi,
-                                            float4 vi, int i, float4* __restrict__ xs, int* __restrict__ key,
-                                            int* __restrict__ rank, int* __restrict__ count,
-                                            int* __restrict__ cellk, int* __restrict__ tile_count) {
+__device__ __forceinline__ int predict_one(const StepParams& p, const CellPack& cp, const Geo& g, float4 xi,
+                                           float4 vi, int i, float4* __restrict__ xs, int* __restrict__ key,
+                                           int* __restrict__ rank, int* __restrict__ count,
+                                           int* __restrict__ cellk) {
     vi.x = __fmaf_rn(p.gxv, p.dt, vi.x);
     vi.y = __fmaf_rn(p.gyv, p.dt, vi.y);
     vi.z = __fmaf_rn(p.gzv, p.dt, vi.z);
@@ -293,10 +291,49 @@ __device__ __forceinline__ void predict_one(const StepParams& p, const CellPack&
     const int k = cell_key(p, cp, g, c, cellk, i);
     key[i] = k;
     rank[i] = atomicAdd(&count[k], 1);
-    if (tile_count) {
-        const int tile = k >> CELL_TILE_SHIFT;
-        const unsigned peers = __match_any_sync(__activemask(), tile);
-        if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&tile_count[tile], __popc(peers));
+    return k;
+}
+
+// The cell scan's per-tile totals, counted with one atomic per tile that the
+// warp's particles fall in (the on-chip solve, whose CTAs work on few tiles each).
+__device__ __forceinline__ void add_tile_warp(int* __restrict__ tile_count, int k) {
+    const int tile = k >> CELL_TILE_SHIFT;
+    const unsigned peers = __match_any_sync(__activemask(), tile);
+    if ((int)(threadIdx.x & 31) == __ffs((int)peers) - 1) atomicAdd(&tile_count[tile], __popc(peers));
+}
+
+// The same by the per-stage prediction.  A tile of CELL_TILE cells holds some
+// thousand particles, which are in flight at the same time (slots are in cell
+// order): an atomic per warp queues them up on a few cache lines (2 M
+// particles: the commit kernel 73 us with one, 62 like this, 58 without totals;
+// the prediction kernel 33 and 25).  A block counts its keys in one
+// tile in shared memory and its last warp adds the sum, one atomic a block;
+// keys of other tiles go to global memory at once.
+struct TileSum {
+    int tile;      // the block's tile
+    unsigned sum;  // its keys << 8 | warps that have counted
+};
+// One thread, before a barrier of the block.
+__device__ __forceinline__ void open_tile_sum(TileSum& t, int key) {
+    t.tile = key >> CELL_TILE_SHIFT;
+    t.sum = 0u;
+}
+// Key k of element i, by every thread of the block whose element is below n
+// (thread t holds element i - threadIdx.x + t).
+__device__ __forceinline__ void add_tile(TileSum& t, int* __restrict__ tile_count, int k, int i, int n) {
+    const int lane = threadIdx.x & 31;
+    const int in_warp = min(32, n - (i - lane)), in_block = min((int)blockDim.x, n - (i - (int)threadIdx.x));
+    const unsigned mask = in_warp == 32 ? 0xffffffffu : (1u << in_warp) - 1u;
+    const int tile = k >> CELL_TILE_SHIFT;
+    const unsigned here = __ballot_sync(mask, tile == t.tile);
+    if (lane == 0) {
+        const unsigned add = ((unsigned)__popc(here) << 8) | 1u, before = atomicAdd(&t.sum, add);
+        if ((before & 0xFFu) == (unsigned)((in_block + 31) / 32 - 1))
+            atomicAdd(&tile_count[t.tile], (int)((before + add) >> 8));
+    }
+    if (tile != t.tile) {
+        const unsigned peers = __match_any_sync(mask & ~here, tile);
+        if (lane == __ffs((int)peers) - 1) atomicAdd(&tile_count[tile], __popc(peers));
     }
 }
 

@@ -43,10 +43,15 @@ __global__ void k_predict(StepParams p, CellPack cp, const float4* __restrict__ 
                           const float4* __restrict__ v, float4* __restrict__ xs, int* __restrict__ key,
                           int* __restrict__ rank, int* __restrict__ count, int* __restrict__ cellk,
                           int* __restrict__ tile_count) {
+    __shared__ TileSum tiles;
     pdl_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= p.n) return;
-    predict_one<MIXED>(p, cp, geo_slot(p, i), x[i], v[i], i, xs, key, rank, count, cellk, tile_count);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = i < p.n;
+    int k = 0;
+    if (live) k = predict_one<MIXED>(p, cp, geo_slot(p, i), x[i], v[i], i, xs, key, rank, count, cellk);
+    if (threadIdx.x == 0) open_tile_sum(tiles, k);
+    __syncthreads();
+    if (live) add_tile(tiles, tile_count, k, i, p.n);
 }
 
 // Cell key and histogram of static particles (solids; scene from solid_scene_of).
@@ -876,16 +881,24 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     static_assert(!COMPACT || (!MIXED && !SOL), "compact lists");
     pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
-    if (MIXED) fill_shift_table(p, shift_tab);
+    __shared__ TileSum tiles;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= p.n) return;
-    const float4 self = xs[s];
-    const float4 vi = v_in[s];
+    const bool live = s < p.n;
+    const float4 self = xs[live ? s : 0];  // in flight across the barrier
+    const float4 vi = v_in[live ? s : 0];
+    const uint4 rec = COMPACT ? __ldg(&p.rec[live ? s : 0]) : make_uint4(0u, 0u, 0u, 0u);
+    // the block's tile: that of its first particle's cell in this step
+    if (xs_next && threadIdx.x == 0) open_tile_sum(tiles, __ldg(&key_sorted[s]));
+    if (MIXED)
+        fill_shift_table(p, shift_tab);
+    else if (xs_next)
+        __syncthreads();
+    if (!live) return;
     const int* __restrict__ col = nbr + s;
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
     if (COMPACT && p.c_xsph != 0.0f) {
         walk_compact<U, WIDE, PosVel>(
-            p, __ldg(&p.rec[s]), p.rec2 + s, col, [&](int t) { return PosVel{xs[t], v_in[t]}; },
+            p, rec, p.rec2 + s, col, [&](int t) { return PosVel{xs[t], v_in[t]}; },
             [&](int t, const PosVel& q) { xsph_pair<false>(p, self, vi, q.x, q.v, t, shift_tab, ax, ay, az); });
     } else if (p.c_xsph != 0.0f) {
         const int c = cnt[s];
@@ -911,7 +924,7 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     const float cx = __fmul_rn(p.c_xsph, p.k6);
     const float4 vc = make_float4(__fmaf_rn(cx, ax, vi.x), __fmaf_rn(cx, ay, vi.y), __fmaf_rn(cx, az, vi.z), 0.0f);
     v_out[s] = vc;
-    const Geo g = (COMPACT && !WIDE) ? geo_of(p, scene_of_record(p, __ldg(reinterpret_cast<const unsigned*>(p.rec + s))))
+    const Geo g = (COMPACT && !WIDE) ? geo_of(p, scene_of_record(p, rec.x))
                                      : geo_slot(p, s);
     float4 xc;
     if (!MIXED && !p.frame) {
@@ -927,10 +940,12 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     }
     x_out[s] = xc;
     if (xs_next) {
+        int k;
         if (MIXED || p.frame)
-            predict_one<true>(p, cp, g, xc, vc, s, xs_next, key, rank, count, cellk, tile_count);
+            k = predict_one<true>(p, cp, g, xc, vc, s, xs_next, key, rank, count, cellk);
         else
-            predict_one<false>(p, cp, g, xc, vc, s, xs_next, key, rank, count, cellk, tile_count);
+            k = predict_one<false>(p, cp, g, xc, vc, s, xs_next, key, rank, count, cellk);
+        add_tile(tiles, tile_count, k, s, p.n);
     }
 }
 

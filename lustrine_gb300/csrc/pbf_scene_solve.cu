@@ -349,8 +349,8 @@ __global__ void __launch_bounds__(T, 1) k_scene_solve(StepParams p, CellPack cp,
             a.x_out[s] = xc;
             a.v_out[s] = vc;
             if (a.xs_next)
-                predict_one<MIXED>(p, cp, sv.g, xc, vc, s, a.xs_next, a.key, a.rank, a.count, a.cellk,
-                                   a.tile_count);
+                add_tile_warp(a.tile_count,
+                              predict_one<MIXED>(p, cp, sv.g, xc, vc, s, a.xs_next, a.key, a.rank, a.count, a.cellk));
         }
         cluster.sync();  // the bin's shared memory is free again
     }

@@ -158,18 +158,25 @@ __global__ void __launch_bounds__(HOST_BLOCK) k_pack_predict(StepParams p, CellP
                                                              int* __restrict__ rank, int* __restrict__ count,
                                                              int* __restrict__ cellk, int* __restrict__ tile_count) {
     __shared__ float sx[3 * HOST_BLOCK], sv[3 * HOST_BLOCK];
+    __shared__ TileSum tiles;
     host_to_smem(hx, n, sx);
     if (hv) host_to_smem(hv, n, sv);
     __syncthreads();
     const int i = blockIdx.x * HOST_BLOCK + threadIdx.x;
-    if (i >= n) return;
-    const int t = 3 * threadIdx.x;
-    const Geo g = geo_single(p);
-    const float4 xi = pack_position<MIXED>(p, cp, g, sx[t], sx[t + 1], sx[t + 2]);
-    const float4 vi = hv ? make_float4(sv[t], sv[t + 1], sv[t + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    x[i] = xi;
-    id[i] = i;
-    predict_one<MIXED>(p, cp, g, xi, vi, i, xs, key, rank, count, cellk, tile_count);
+    const bool live = i < n;
+    int k = 0;
+    if (live) {
+        const int t = 3 * threadIdx.x;
+        const Geo g = geo_single(p);
+        const float4 xi = pack_position<MIXED>(p, cp, g, sx[t], sx[t + 1], sx[t + 2]);
+        const float4 vi = hv ? make_float4(sv[t], sv[t + 1], sv[t + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        x[i] = xi;
+        id[i] = i;
+        k = predict_one<MIXED>(p, cp, g, xi, vi, i, xs, key, rank, count, cellk);
+    }
+    if (threadIdx.x == 0) open_tile_sum(tiles, k);
+    __syncthreads();
+    if (live) add_tile(tiles, tile_count, k, i, n);
 }
 
 __global__ void k_slot_of(const int* __restrict__ id, int n, int* __restrict__ slot_of) {
