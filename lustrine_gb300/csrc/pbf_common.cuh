@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
 #include <utility>
 
 namespace lgb {
@@ -52,15 +53,22 @@ struct SceneInfo {
 constexpr int COMPACT_INLINE = 6;
 constexpr int COMPACT_EXT = 8;
 constexpr int COMPACT_RECORDS = COMPACT_INLINE + COMPACT_EXT;
-// Wide records (StepParams::wide): record.x = count; .y, .z, .w = entries
-// 0-2 as slots (the sentinel slot n past the count); the second record,
-// entries 3-6.
+// Larger scenes (StepParams::wide): slots, the sentinel slot n past the count.
+// Contexts of fewer than COMPACT_MAX_N particles take 24-bit slots (wide 1):
+// record.x = count | entry 0 << 8; .y, .z, .w = entries 1-3 in their low 24
+// bits and entry 4 in their high bytes; the second record, entries 5-8 in the
+// low 24 bits and entry 9 in the high bytes of .x, .y, .z.  Others 32-bit
+// slots (wide 2): record.x = count; .y, .z, .w = entries 0-2; the second
+// record, entries 3-6.  (2 M particles, 4 neighbours each: half the lists are
+// longer than 3, one in seven longer than 5.)
+constexpr int WIDE24_INLINE = 5;
+constexpr int WIDE24_EXT = 5;
 constexpr int WIDE_INLINE = 3;
 constexpr int WIDE_EXT = 4;
 constexpr int WIDE_RECORDS = WIDE_INLINE + WIDE_EXT;
 constexpr unsigned COMPACT_SENTINEL = 0xFFFFu;
 constexpr int COMPACT_MAX_SCENE = 65535;   // scene-local offsets 0..65534
-constexpr int COMPACT_MAX_N = 1 << 24;     // first slot in 24 bits
+constexpr int COMPACT_MAX_N = 1 << 24;     // first slot (or slots) in 24 bits
 constexpr int COMPACT_MAX_NBRS = 255;      // count in 8 bits
 
 // Everything a step kernel reads, passed by value (constant bank).
@@ -106,7 +114,7 @@ struct StepParams {
     int frame;            // mixed storage, iterations in the scene frame (LUSTRINE_PRECISION_MIXED_SCENE)
     uint4* rec;           // compact neighbour lists of this step (nullptr: column lists with counts)
     uint4* rec2;          // their second records
-    int wide;             // compact lists in wide records (32-bit slots)
+    int wide;             // compact lists in wide records: 1 24-bit slots, 2 32-bit slots (0: 16-bit offsets)
     const int* src;       // the previous slot of each sorted slot, whose committed position the last
                           // position pass reads from the unsorted state (nullptr: sorted with the step)
 };
@@ -153,6 +161,11 @@ __device__ __forceinline__ float hi2(f32x2 a) { return __uint_as_float((unsigned
 __device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) {
     f32x2 r;
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
     return r;
 }
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
@@ -206,6 +219,9 @@ bool pdl_enabled();
 // PBF neighbour lists: rows allocated = max_nbrs rounded up to LIST_PAD_MAX;
 // the sentinel slot n sits at SENTINEL_POS on every axis.
 constexpr int LIST_PAD_MAX = 8;
+// Column lists: the bit of a particle's count that says that its list holds
+// static particles.
+constexpr int CNT_SOLID = 1 << 30;
 constexpr float SENTINEL_POS = 1e18f;
 // The list builds load candidates in chunks that may reach past a cell
 // range's end: position buffers are this much longer than their particles.

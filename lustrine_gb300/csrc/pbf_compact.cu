@@ -21,19 +21,28 @@ void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4
         else if (B == 128) LGB_LISTS_C(H, FR, W, 128); \
         else LGB_LISTS_C(H, FR, W, 256);              \
     } while (0)
-    if (p.frame && p.wide) LGB_LISTS_CB(false, true, true);
-    else if (p.frame) LGB_LISTS_CB(false, true, false);
-    else if (p.hash_bits && p.wide) LGB_LISTS_CB(true, false, true);
-    else if (p.hash_bits) LGB_LISTS_CB(true, false, false);
-    else if (p.wide) LGB_LISTS_CB(false, false, true);
-    else LGB_LISTS_CB(false, false, false);
+#define LGB_LISTS_CW(H, FR)                           \
+    do {                                              \
+        if (p.wide == 2) LGB_LISTS_CB(H, FR, L_C32);  \
+        else if (p.wide) LGB_LISTS_CB(H, FR, L_C24);  \
+        else LGB_LISTS_CB(H, FR, L_C16);              \
+    } while (0)
+    if (p.frame) LGB_LISTS_CW(false, true);
+    else if (p.hash_bits) LGB_LISTS_CW(true, false);
+    else LGB_LISTS_CW(false, false);
+#undef LGB_LISTS_CW
 #undef LGB_LISTS_CB
 #undef LGB_LISTS_C
 }
 
-// fcode of a compact pass: 8, | 16 for wide records; the lambda pass | 4 in
-// the scene frame
-static int compact_fcode(const StepParams& p) { return 8 | (p.wide ? 16 : 0); }
+// fcode of a compact pass: 8, | 16 for 24-bit records, | 32 for 32-bit ones
+// (ListFormatOf); the lambda pass | 4 in the scene frame
+static int compact_fcode(const StepParams& p) { return 8 | (p.wide == 2 ? 32 : (p.wide ? 16 : 0)); }
+
+// Contexts of 2^24 particles and more: the passes of 32-bit records come in
+// one shape, the best one of large scenes.
+#define LGB_ONE_SHAPE(KERNEL, FF, ...) \
+    launch_k(KERNEL<FF, 1, 256>, blocks_for(p.n, 256), 256, st, pdl_enabled(), __VA_ARGS__)
 
 void launch_lambda_compact(const Tuning& tu, const StepParams& p, float4* xs, const int* nbr, const int* cnt,
                            const float4* solid, float* rho, cudaStream_t st) {
@@ -41,7 +50,9 @@ void launch_lambda_compact(const Tuning& tu, const StepParams& p, float4* xs, co
         case 8: TUNE_CASE(k_lambda, 8, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
         case 12: TUNE_CASE(k_lambda, 12, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
         case 24: TUNE_CASE(k_lambda, 24, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
-        default: TUNE_CASE(k_lambda, 28, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
+        case 28: TUNE_CASE(k_lambda, 28, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
+        case 40: LGB_ONE_SHAPE(k_lambda, 40, p, xs, nbr, cnt, solid, rho); break;
+        default: LGB_ONE_SHAPE(k_lambda, 44, p, xs, nbr, cnt, solid, rho); break;
     }
 }
 
@@ -50,7 +61,8 @@ void launch_delta_compact(const Tuning& tu, const StepParams& p, const CellPack&
                           const int* key_sorted, const float4* x, float4* v_out, cudaStream_t st) {
     switch (compact_fcode(p)) {
         case 8: TUNE_CASE(k_delta, 8, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
-        default: TUNE_CASE(k_delta, 24, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
+        case 24: TUNE_CASE(k_delta, 24, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
+        default: LGB_ONE_SHAPE(k_delta, 40, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
     }
 }
 
@@ -59,6 +71,11 @@ void launch_xsph_compact(const Tuning& tx, const StepParams& p, const CellPack& 
                          float4* v_out, float4* xs_next, int* key, int* rank, int* count, int* cellk,
                          int* tile_count, cudaStream_t st) {
     const int f = compact_fcode(p);
+    if (f == 40) {
+        LGB_ONE_SHAPE(k_xsph_compact, 40, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next, key, rank,
+                      count, cellk, tile_count);
+        return;
+    }
     if (tx.unroll <= 1) {  // the 32-register kernel, one gather in flight
         const int B = tx.block <= 64 ? 64 : (tx.block <= 128 ? 128 : 256);
 #define LGB_XC(FF, BB)                                                                                  \

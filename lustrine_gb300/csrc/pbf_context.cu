@@ -1009,7 +1009,8 @@ static int enqueue_step(lustrine_pbf* s, cudaStream_t st, StageMarks* mk = nullp
         s->lists_format = compact_now(s);
         pl.rec = s->lists_format != LUSTRINE_LISTS_COLUMN ? s->rec : nullptr;
         pl.rec2 = pl.rec ? s->rec2 : nullptr;
-        pl.wide = s->lists_format == LUSTRINE_LISTS_COMPACT_WIDE;
+        pl.wide = s->lists_format != LUSTRINE_LISTS_COMPACT_WIDE ? 0 : (s->cap < COMPACT_MAX_N ? 1 : 2);
+        s->lists_wide = pl.wide;
         pl.src = s->src;
         float4* a = s->xs[o];
         float4* b = s->xs_alt;
@@ -1569,24 +1570,29 @@ extern "C" int lustrine_pbf_neighbors(lustrine_pbf* s, int* count, int* idx, int
     CK(cudaStreamSynchronize(s->stream));
     if (compact) {
         // compact records into the column form: count, the records' entries
-        // (16-bit: the scene's first slot + offset; wide: the slot; the
-        // second record is written only for lists longer than its first),
-        // the rest from the overflow rows
-        const bool wide = s->lists_format == LUSTRINE_LISTS_COMPACT_WIDE;
-        const int R = wide ? WIDE_RECORDS : COMPACT_RECORDS;
+        // (the second record is written only for lists longer than the
+        // first holds), the rest from the overflow rows
+        const int wide = s->lists_wide;
+        const int R = wide == 2 ? WIDE_RECORDS : (wide ? WIDE24_INLINE + WIDE24_EXT : COMPACT_RECORDS);
         std::vector<int> col((size_t)maxn * n);
         for (int k = 0; k < n; k++) {
             const uint4 r = rec[(size_t)k], x = rec2[(size_t)k];
-            const unsigned w[7] = {r.y, r.z, r.w, x.x, x.y, x.z, x.w};
-            const int c = wide ? (int)r.x : (int)(r.x & 0xFFu), base = wide ? 0 : (int)(r.x >> 8);
+            const unsigned w[8] = {r.x, r.y, r.z, r.w, x.x, x.y, x.z, x.w};
+            const int c = wide == 2 ? (int)r.x : (int)(r.x & 0xFFu);
+            auto high = [&](int a) { return (int)((w[a] >> 24) | (w[a + 1] >> 24 << 8) | (w[a + 2] >> 24 << 16)); };
+            auto entry = [&](int e) {
+                if (wide == 2) return (int)w[e + 1];
+                if (wide) return e == 0 ? (int)(w[0] >> 8) : (e == 4 ? high(1) : (e == 9 ? high(4)
+                                                                      : (int)(w[e < 5 ? e : e - 1] & 0xFFFFFFu)));
+                return (int)(r.x >> 8) + (int)((w[1 + (e >> 1)] >> ((e & 1) * 16)) & 0xFFFFu);
+            };
             cnt[(size_t)k] = c;
-            for (int e = 0; e < c; e++)
-                col[(size_t)e * n + k] = e >= R ? nbr[(size_t)(e - R) * n + k]
-                                         : wide ? (int)w[e]
-                                                : base + (int)((w[e >> 1] >> ((e & 1) * 16)) & 0xFFFFu);
+            for (int e = 0; e < c; e++) col[(size_t)e * n + k] = e >= R ? nbr[(size_t)(e - R) * n + k] : entry(e);
         }
         nbr.swap(col);
     }
+    if (s->prm.mode == LUSTRINE_MODE_PBF)
+        for (int& c : cnt) c &= ~CNT_SOLID;
     int rc = LUSTRINE_OK;
     // reference-semantics lists: slot t >= 0 or static slot -1 - u; the sand
     // lists leave the particle itself out (the reference lists it twice)

@@ -71,6 +71,7 @@ struct lustrine_pbf {
     uint4* rec2 = nullptr;       // their second records
     int* src = nullptr;          // PBF step: previous slot of each sorted slot (its committed position)
     int lists_format = LUSTRINE_LISTS_COLUMN;  // the form the last list build wrote (LUSTRINE_LISTS_*)
+    int lists_wide = 0;          // its records: StepParams::wide
     float* lam = nullptr;
     float4* lam_src = nullptr;  // PBF: the buffer whose w holds the last lambdas
     float* lam_by_id = nullptr;

@@ -96,286 +96,317 @@ __global__ void k_mark_solid_near(StepParams p, CellPack cp, const float4* __res
             }
 }
 
-// Where the list build puts a particle's entries.  Column lists: entry k of
-// slot s at nbr[k * n + s] with its cell codes and solid flag.
-struct ColumnLists {
-    int* nbr;
-    int n, s;
-    __device__ __forceinline__ void put(int k, int t, int dx, int dy, int dz, bool solid) {
-        nbr[(size_t)k * n + s] = entry(t, dx, dy, dz, solid);
-    }
-};
+// List formats: column lists, or compact lists in one of three records
+// (CompactLists in pbf_common.cuh): 16-bit offsets from the scene's first slot,
+// 24-bit slots, 32-bit slots.
+enum : int { L_COLUMN = 0, L_C16 = 1, L_C24 = 2, L_C32 = 3 };
 
 // Entries a compact list keeps in its two records: inline (first record),
 // second record, both.
-template <bool WIDE>
+template <int FMT>
 struct RecordFormat {
-    static constexpr int INLINE = WIDE ? WIDE_INLINE : COMPACT_INLINE;
-    static constexpr int EXT = WIDE ? WIDE_EXT : COMPACT_EXT;
+    static constexpr int INLINE = FMT == L_C16 ? COMPACT_INLINE : (FMT == L_C24 ? WIDE24_INLINE : WIDE_INLINE);
+    static constexpr int EXT = FMT == L_C16 ? COMPACT_EXT : (FMT == L_C24 ? WIDE24_EXT : WIDE_EXT);
     static constexpr int RECORDS = INLINE + EXT;
 };
 
-// Compact lists: the records' entries (16-bit offsets from the scene's
-// first slot, or 32-bit slots in wide records) staged in the thread's
-// COMPACT_STRIDE words of shared memory (filled with the sentinel first; a
-// stride of 9 words keeps a warp's stores and loads free of bank conflicts)
-// until the records are written; the rest as plain slots in the column rows
-// of nbr from row 0.  No cell codes and no static particles (the step uses
-// compact lists only without either).
+// The high bytes of three words as a 24-bit value, and a 24-bit value's byte b
+// as a word's high byte: where a 24-bit record keeps its fifth entry.
+__device__ __forceinline__ int high_bytes(unsigned a, unsigned b, unsigned c) {
+    return (int)__byte_perm(__byte_perm(a, b, 0x0073), c >> 24, 0x5410);
+}
+__device__ __forceinline__ unsigned as_high_byte(unsigned e, int b) { return (e >> (8 * b)) << 24; }
+
+// Entry k of a record (FIRST: the first, else the second); 16-bit records:
+// the offset.
+template <int FMT, bool FIRST>
+__device__ __forceinline__ unsigned record_entry(const uint4& r, int k) {
+    constexpr unsigned M = 0xFFFFFFu;
+    if (FMT == L_C24) {
+        if (FIRST)
+            return k == 0 ? r.x >> 8 : (k == 1 ? r.y & M : (k == 2 ? r.z & M : (k == 3 ? r.w & M
+                                                                                        : (unsigned)high_bytes(r.y, r.z, r.w))));
+        return k == 0 ? r.x & M : (k == 1 ? r.y & M : (k == 2 ? r.z & M : (k == 3 ? r.w
+                                                                                  : (unsigned)high_bytes(r.x, r.y, r.z))));
+    }
+    const int j = (FMT == L_C16 ? k >> 1 : k) + (FIRST ? 1 : 0);  // the word
+    const unsigned x = j == 0 ? r.x : (j == 1 ? r.y : (j == 2 ? r.z : r.w));
+    if (FMT == L_C32) return x;
+    return (k & 1) ? x >> 16 : x & 0xFFFFu;
+}
+
+// A thread's list while the stencil is walked: column lists (entry k of slot s
+// at nbr[k n + s] with its cell codes and solid flag) or compact lists.  The
+// first CAP accepted entries wait in shared memory, the 32-bit ones with entry
+// k at [k][thread]; the 16-bit ones take COMPACT_STRIDE consecutive words a
+// thread (an odd stride: no bank conflicts among equal k), read back as the
+// records' words.  Entries past CAP go to their rows of nbr at once.
+// STAGED (column lists on a dense grid): a candidate costs one store to the next
+// free place and a conditional step of the pointer, a refused one overwritten
+// by the next, where a store under a branch runs the branch for the warp
+// whenever a lane accepts.  That pays for rows of several particles a cell
+// (262,144 particles on voxels, 1.6 a cell: 35.5 us with the first lambda
+// summed in the branch, 31.9 like this, 32.2 with the store in it), not for
+// compact lists at unit density (2 M particles: 105 against 101 us) or one-cell
+// buckets (1 M particles hashed: 183 against 177 us).
 constexpr int COMPACT_STRIDE = 9;
-template <bool WIDE>
-struct CompactLists {
-    int* ovf;
-    int n, s, base;
-    unsigned* stage;  // this thread's words
-    __device__ __forceinline__ void put(int k, int t, int, int, int, bool) {
-        constexpr int R = RecordFormat<WIDE>::RECORDS;
-        if (k >= R)
-            ovf[(size_t)(k - R) * n + s] = t;
-        else if (WIDE)
-            stage[k] = (unsigned)t;
+template <int FORMAT, int B, bool STAGED>
+struct StagedEntries {
+    static constexpr int CAP = FORMAT == L_C16 ? 2 * COMPACT_STRIDE : 16;
+    static constexpr int WORDS = FORMAT == L_C16 ? COMPACT_STRIDE * B : CAP * B;  // of the block
+    static constexpr int STEP = FORMAT == L_C16 ? 1 : B;
+    static constexpr int ROW0 = FORMAT == L_COLUMN ? 0 : RecordFormat<FORMAT>::RECORDS;  // entry of nbr's row 0
+    using T = typename std::conditional<FORMAT == L_C16, unsigned short, int>::type;
+    T* first;  // entry 0
+    T* at;     // the next place
+    int* row;  // nbr + s
+    int base;  // 16-bit entries: the scene's first slot
+    int extra = 0;  // entries past CAP
+    __device__ __forceinline__ StagedEntries(unsigned* smem, int* nbr, const StepParams& p, int s, int slot0)
+        : row(nbr + s), base(slot0) {
+        if (FORMAT == L_C16)
+            first = reinterpret_cast<T*>(smem + COMPACT_STRIDE * threadIdx.x);
         else
-            reinterpret_cast<unsigned short*>(stage)[k] = (unsigned short)(t - base);
-    }
-    // entry k < count of the list put so far (the thread reads back its own stores)
-    __device__ __forceinline__ int get(int k) const {
-        constexpr int R = RecordFormat<WIDE>::RECORDS;
-        if (k >= R) return ovf[(size_t)(k - R) * n + s];
-        if (WIDE) return (int)stage[k];
-        return base + reinterpret_cast<const unsigned short*>(stage)[k];
-    }
-};
-
-// 0: column lists; 1: compact; 2: compact in wide records
-template <int FORMAT>
-struct ListsOf {
-    using T = ColumnLists;
-};
-template <>
-struct ListsOf<1> {
-    using T = CompactLists<false>;
-};
-template <>
-struct ListsOf<2> {
-    using T = CompactLists<true>;
-};
-__device__ __forceinline__ ColumnLists open_lists(ColumnLists*, int* nbr, int n, int s, int, unsigned*) {
-    return ColumnLists{nbr, n, s};
-}
-template <bool WIDE>
-__device__ __forceinline__ CompactLists<WIDE> open_lists(CompactLists<WIDE>*, int* nbr, int n, int s, int base,
-                                                         unsigned* stage) {
-    unsigned* mine = stage + COMPACT_STRIDE * threadIdx.x;
-    if (WIDE) {
+            first = reinterpret_cast<T*>(smem) + threadIdx.x;
+        at = first;
+        // places past the count hold the sentinel in the records
+        if (FORMAT == L_C16) {
 #pragma unroll
-        for (int q = 0; q < WIDE_RECORDS; q++) mine[q] = (unsigned)n;
-    } else {
+            for (int q = 0; q < COMPACT_RECORDS / 2; q++) reinterpret_cast<unsigned*>(first)[q] = 0xFFFFFFFFu;
+        } else {
 #pragma unroll
-        for (int q = 0; q < COMPACT_RECORDS / 2; q++) mine[q] = 0xFFFFFFFFu;
-    }
-    return CompactLists<WIDE>{nbr, n, s, base, mine};
-}
-// The count and the sentinel entries up to a multiple of the passes' chunk
-// (pad divides the buffer's rows: max_nbrs rounded up to LIST_PAD_MAX).
-__device__ __forceinline__ void close_lists(const StepParams& p, const ColumnLists& l, int* __restrict__ cnt,
-                                            int c_n) {
-    cnt[l.s] = c_n;
-    for (int k = c_n; k % p.pad != 0; k++) l.nbr[(size_t)k * p.n + l.s] = sentinel_entry(p);
-}
-template <bool WIDE>
-__device__ __forceinline__ void close_lists(const StepParams& p, const CompactLists<WIDE>& l, int*, int c_n) {
-    using RF = RecordFormat<WIDE>;
-    const unsigned* w = l.stage;
-    const unsigned head = WIDE ? (unsigned)c_n : ((unsigned)c_n | ((unsigned)l.base << 8));
-    p.rec[l.s] = make_uint4(head, w[0], w[1], w[2]);
-    if (c_n > RF::INLINE) p.rec2[l.s] = make_uint4(w[3], w[4], w[5], w[6]);
-    for (int k = c_n - RF::RECORDS; k > 0 && k % p.pad != 0; k++) l.ovf[(size_t)k * p.n + l.s] = p.n;
-}
-
-// A candidate within h, the c_n-th accepted.  PH 0: listed (below the
-// capacity) and summed into the first lambda; PH 1: listed only (the sums
-// run over the list afterwards); PH 2: summed only if past the capacity (the
-// entries the list dropped, after the listed ones' sums).
-template <int PH, bool KAHAN, bool SOLID, class L>
-__device__ __forceinline__ void accept(const StepParams& p, LambdaAcc& a, const float3& d, int& c_n, L& out, int t,
-                                       int dx, int dy, int dz) {
-    if (PH != 2 && c_n < p.max_nbrs) out.put(c_n, t, dx, dy, dz, SOLID);
-    if (PH == 0 || (PH == 2 && c_n >= p.max_nbrs)) lambda_accumulate<KAHAN>(p, a, d, SOLID);
-    c_n++;
-}
-
-// One row (dy, dx) of the stencil: the cells z0..z1 of a row are consecutive
-// ids, so their particles form one slot range, walked in one loop (a warp
-// then runs as many rounds as its fullest row, not the sum over the three
-// cells of its fullest cell); a candidate's dz follows from the cell bounds,
-// loaded once per row.  The candidates come in the same order as cell by cell.
-template <bool MIXED, bool SOLID, bool KAHAN, class L, int PH = 0>
-__device__ __forceinline__ void walk_row(const StepParams& p, const float4& self, int s,
-                                         const float4* __restrict__ pos, const int* __restrict__ start,
-                                         int row, int zc, int gz, int dx, int dy, LambdaAcc& a, int& c_n,
-                                         L& out) {
-    const int z0 = max(zc - 1, 0), z1 = min(zc + 1, gz - 1);
-    const int b0 = start[row + z0];
-    const int b1 = start[row + z0 + 1];
-    const int b2 = (z0 + 1 <= z1) ? start[row + z0 + 2] : b1;
-    const int b3 = (z0 + 2 <= z1) ? start[row + z0 + 3] : b2;
-    const int dz0 = z0 - zc;
-    const float sx = -(float)dx * p.cell, sy = -(float)dy * p.cell;
-    for (int t = b0; t < b3; t++) {
-        if (!SOLID && t == s) continue;
-        const int dz = dz0 + (t >= b1) + (t >= b2);
-        const float4 q = SOLID ? __ldg(&pos[t]) : pos[t];
-        float3 d = make_float3(__fsub_rn(self.x, q.x), __fsub_rn(self.y, q.y), __fsub_rn(self.z, q.z));
-        if (MIXED) {
-            d.x = __fadd_rn(d.x, sx);
-            d.y = __fadd_rn(d.y, sy);
-            d.z = __fadd_rn(d.z, -(float)dz * p.cell);
+            for (int q = 0; q < ROW0; q++) first[q * STEP] = (T)p.n;
         }
-        if (dot3e(d.x, d.y, d.z) <= p.h2) accept<PH, KAHAN, SOLID>(p, a, d, c_n, out, t, dx, dy, dz);
     }
+    __device__ __forceinline__ bool room(int w) const { return at <= first + (CAP - w) * STEP; }
+    __device__ __forceinline__ void put(int e, bool in) {  // with room only
+        *at = (T)(FORMAT == L_C16 ? e - base : e);
+        at += in ? STEP : 0;
+    }
+    __device__ __forceinline__ void push(const StepParams& p, int e) {
+        if (at < first + CAP * STEP) {
+            put(e, true);
+        } else {
+            if (CAP + extra < p.max_nbrs) row[(size_t)(CAP - ROW0 + extra) * p.n] = e;
+            extra++;
+        }
+    }
+    template <int W>
+    __device__ __forceinline__ void take(const StepParams& p, const int (&e)[W], const bool (&in)[W]) {
+        if (STAGED && room(W)) {
+#pragma unroll
+            for (int u = 0; u < W; u++) put(e[u], in[u]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < W; u++)
+                if (in[u]) push(p, e[u]);
+        }
+    }
+    __device__ __forceinline__ int staged() const { return (int)(at - first) / STEP; }
+    __device__ __forceinline__ int count() const { return staged() + extra; }
+    // entry k below the count and the capacity
+    __device__ __forceinline__ int get(const StepParams& p, int k) const {
+        if (k >= CAP) return row[(size_t)(k - ROW0) * p.n];
+        return (FORMAT == L_C16 ? base : 0) + (int)first[k * STEP];
+    }
+    // The list's c_n entries: records and rows, and the rows' sentinel entries
+    // up to a multiple of the passes' chunk (pad divides the buffer's rows:
+    // max_nbrs rounded up to LIST_PAD_MAX).  solid: a column list holds some.
+    __device__ __forceinline__ void close(const StepParams& p, int s, int* __restrict__ cnt, int c_n, bool solid) {
+        const int m = min(staged(), c_n);
+        if (FORMAT == L_COLUMN) {
+            cnt[s] = c_n | (solid ? CNT_SOLID : 0);
+            for (int k = 0; k < m; k++) row[(size_t)k * p.n] = (int)first[k * STEP];
+            for (int k = c_n; k % p.pad != 0; k++) row[(size_t)k * p.n] = sentinel_entry(p);
+            return;
+        }
+        for (int k = ROW0; k < m; k++) row[(size_t)(k - ROW0) * p.n] = get(p, k);
+        // places from the count on: the last refused candidate's, or entries
+        // cut at the capacity
+        for (int k = m; k < min(staged() + 1, ROW0); k++) first[k * STEP] = (T)(FORMAT == L_C16 ? 0xFFFF : p.n);
+        uint4 r, r2;
+        if (FORMAT == L_C16) {
+            const unsigned* w = reinterpret_cast<const unsigned*>(first);
+            r = make_uint4((unsigned)c_n | ((unsigned)base << 8), w[0], w[1], w[2]);
+            r2 = make_uint4(w[3], w[4], w[5], w[6]);
+        } else {
+            auto e = [&](int k) { return (unsigned)first[k * STEP]; };
+            if (FORMAT == L_C24) {
+                r = make_uint4((unsigned)c_n | (e(0) << 8), e(1) | as_high_byte(e(4), 0), e(2) | as_high_byte(e(4), 1),
+                               e(3) | as_high_byte(e(4), 2));
+                r2 = make_uint4(e(5) | as_high_byte(e(9), 0), e(6) | as_high_byte(e(9), 1),
+                                e(7) | as_high_byte(e(9), 2), e(8));
+            } else {
+                r = make_uint4((unsigned)c_n, e(0), e(1), e(2));
+                r2 = make_uint4(e(3), e(4), e(5), e(6));
+            }
+        }
+        p.rec[s] = r;
+        if (c_n > ROW0 - RecordFormat<FORMAT>::EXT) p.rec2[s] = r2;
+        for (int k = c_n - ROW0; k > 0 && k % p.pad != 0; k++) row[(size_t)k * p.n] = p.n;
+    }
+};
+
+// x_i - x_j of a pair from the list entry e of its neighbour q, as the walk formed it.
+template <bool MIXED>
+__device__ __forceinline__ float3 rel_entry(const StepParams& p, const float4& self, const float4& q, int e) {
+    float3 d = make_float3(__fsub_rn(self.x, q.x), __fsub_rn(self.y, q.y), __fsub_rn(self.z, q.z));
+    if (MIXED) {
+        d.x = __fadd_rn(d.x, axis_shift(p.cell, e, 25));
+        d.y = __fadd_rn(d.y, axis_shift(p.cell, e, 27));
+        d.z = __fadd_rn(d.z, axis_shift(p.cell, e, 29));
+    }
+    return d;
 }
 
-// The candidates [t_begin, t_end) of one row, gathered W at a time (the
-// loads of a chunk are in flight together; the tests run in slot order, so
-// the list is the one walk_row builds).  W = 4; the compact list build takes
-// 2 and loads each row's bounds just before the row, for fewer live
-// registers (config 3 lists 0.522 -> 0.493 ms at step 50 of the run, both
-// steps together).  b1, b2: the row's cell bounds, read
-// in mixed precision only (the entry's dz code and the cell shift; fp32
-// entries carry dz = 0, which no fp32 pass reads).
-template <bool MIXED, bool SOLID, bool KAHAN, class L, int W = 4, int PH = 0>
-__device__ __forceinline__ void walk_range(const StepParams& p, const float4& self, int s,
-                                           const float4* __restrict__ pos, int t_begin, int t_end, int b1, int b2,
-                                           int dz0, int dx, int dy, LambdaAcc& a, int& c_n, L& out) {
-    const float sx = -(float)dx * p.cell, sy = -(float)dy * p.cell;
-    for (int t0 = t_begin; t0 < t_end; t0 += W) {
-        float4 q[W];
+// The entries a list dropped at its capacity, summed into the first lambda
+// after the listed ones (a second walk, only where a list was cut).
+template <bool MIXED, bool KAHAN>
+struct DroppedEntries {
+    LambdaAcc& a;
+    const float4& self;
+    const float4* xs;
+    const float4* solid;
+    int c;
+    template <int W>
+    __device__ __forceinline__ void take(const StepParams& p, const int (&e)[W], const bool (&in)[W]) {
 #pragma unroll
         for (int u = 0; u < W; u++)
-            if (t0 + u < t_end) q[u] = SOLID ? __ldg(&pos[t0 + u]) : pos[t0 + u];
+            if (in[u] && c++ >= p.max_nbrs)
+                lambda_accumulate<KAHAN>(p, a, rel_entry<MIXED>(p, self, load_entry(e[u], xs, solid), e[u]),
+                                         entry_solid(e[u]));
+    }
+};
+
+// The candidates [t0, t1) of one stencil row (its three cells' ids are
+// consecutive, so their particles are one slot range), tested in slot order:
+// W positions loaded together (past t1 too: the buffers are SPAN_PAD
+// longer), each within h offered to out.  code: the entry's cell code of the
+// row (dx, dy; dz = 0) and its solid flag; MIXED: b1, b2 are the bounds of the row's
+// second and third cell, which give the entry's dz code and the cell shift.
+// fp32 entries carry dz = 0, which no fp32 pass reads.
+static_assert(4 <= SPAN_PAD, "a range reads at most SPAN_PAD positions past its end");
+template <bool MIXED, int W, class L>
+__device__ __forceinline__ void walk_range(const StepParams& p, const float4& self, int skip, const float4* pos,
+                                           int t0, int t1, int b1, int b2, int dz0, int code, L& out) {
+    for (int t = t0; t < t1; t += W) {
+        float4 q[W];
+        int e[W];
+        bool in[W];
+#pragma unroll
+        for (int u = 0; u < W; u++) q[u] = pos[t + u];
+        const int left = t1 - t, self_at = skip - t;
 #pragma unroll
         for (int u = 0; u < W; u++) {
-            const int t = t0 + u;
-            if (t >= t_end || (!SOLID && t == s)) continue;
-            const int dz = MIXED ? dz0 + (t >= b1) + (t >= b2) : 0;
             float3 d = make_float3(__fsub_rn(self.x, q[u].x), __fsub_rn(self.y, q[u].y), __fsub_rn(self.z, q[u].z));
+            e[u] = t + u + code;
             if (MIXED) {
-                d.x = __fadd_rn(d.x, sx);
-                d.y = __fadd_rn(d.y, sy);
-                d.z = __fadd_rn(d.z, -(float)dz * p.cell);
+                const int cz = dz0 + (t + u >= b1) + (t + u >= b2);
+                e[u] += cz << 29;
+                d.x=__fadd_rn(d.x, axis_shift(p.cell, code, 25)); d.y=__fadd_rn(d.y, axis_shift(p.cell, code, 27));
+                d.z = __fadd_rn(d.z, -(float)cz * p.cell);
             }
-            if (dot3e(d.x, d.y, d.z) <= p.h2) accept<PH, KAHAN, SOLID>(p, a, d, c_n, out, t, dx, dy, dz);
+            in[u] = u < left && u != self_at && dot3e(d.x,d.y,d.z) <= p.h2;
         }
+        out.take(p, e, in);
     }
 }
 
-// One cell of the stencil on a hashed grid: the particles of its bucket,
-// kept only if they belong to that cell.
-template <bool MIXED, bool SOLID, bool KAHAN, class L, int PH = 0>
-__device__ __forceinline__ void walk_hashed_cell(const StepParams& p, const float4& self, int s,
-                                                 const float4* __restrict__ pos,
-                                                 const int* __restrict__ start,
-                                                 const int* __restrict__ cells, int b, int packed,
-                                                 int dx, int dy, int dz, LambdaAcc& a, int& c_n, L& out) {
-    const float sx = -(float)dx * p.cell, sy = -(float)dy * p.cell, sz = -(float)dz * p.cell;
-    for (int t = start[b], e = start[b + 1]; t < e; t++) {
-        if ((!SOLID && t == s) || __ldg(&cells[t]) != packed) continue;
-        const float4 q = SOLID ? __ldg(&pos[t]) : pos[t];
-        float3 d = make_float3(__fsub_rn(self.x, q.x), __fsub_rn(self.y, q.y), __fsub_rn(self.z, q.z));
+// One cell of the stencil on a hashed grid: the particles of its bucket's slots
+// [t0, t1), kept only if they belong to that cell (packed).  code: the entry's
+// cell code and solid flag.  (The paired subtraction and shift keep the build at
+// 48 registers, 1 M particles in 178 us; one axis at a time it took 56 and 201.)
+template <bool MIXED, class L>
+__device__ __forceinline__ void walk_bucket(const StepParams& p, const float4& self, int skip, const float4* pos,
+                                            const int* __restrict__ cells, int packed, int t0, int t1, int code,
+                                            L& out) {
+    const f32x2 sxy = pack2(self.x, self.y);
+    const f32x2 shift = pack2(axis_shift(p.cell, code, 25), axis_shift(p.cell, code, 27));
+    const float shift_z = axis_shift(p.cell, code, 29);
+    for (int t = t0; t < t1; t++) {
+        const ulonglong2 o = reinterpret_cast<const ulonglong2*>(pos)[t];
+        f32x2 dxy = sub2(sxy, o.x);
+        float dz = __fsub_rn(self.z, lo2(o.y));
         if (MIXED) {
-            d.x = __fadd_rn(d.x, sx);
-            d.y = __fadd_rn(d.y, sy);
-            d.z = __fadd_rn(d.z, sz);
+            dxy = add2(dxy, shift);
+            dz = __fadd_rn(dz, shift_z);
         }
-        if (dot3e(d.x, d.y, d.z) <= p.h2) accept<PH, KAHAN, SOLID>(p, a, d, c_n, out, t, dx, dy, dz);
+        const int e[1] = {t + code};
+        const bool in[1] = {t != skip && __ldg(&cells[t]) == packed && dot3e(lo2(dxy), hi2(dxy), dz) <= p.h2};
+        out.take(p, e, in);
     }
 }
 
-// The stencil's candidates of fluid slot s in cell c, in list order: on a
-// dense grid the nine rows (with the static particles of each row after its
-// fluid ones where the neighbourhood holds some); on a hashed grid the
-// cells' buckets.  PH: what each accepted candidate does (accept()).
-template <int PH, bool MIXED, bool HASHED, bool KAHAN, bool COMPACT, class Lists>
+// The stencil's candidates of fluid slot s in cell c, in list order, offered to
+// out: on a dense grid the nine rows (with the static particles of each row
+// after its fluid ones where the neighbourhood holds some, near); on a hashed
+// grid the cells' buckets.  CODES: entries with cell codes (column lists).  A
+// row's bounds are loaded just before its walk (fewer live registers, more
+// resident warps), those of a row's three buckets together.
+template <bool MIXED, bool HASHED, bool SOLIDS, bool CODES, class L>
 __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack& cp, const float4& self, int s,
-                                             const int3& c, const Geo& g, const float4* __restrict__ xs,
+                                             const int3& c, const Geo& g, const float4* xs,
                                              const int* __restrict__ cell_sorted, const int* __restrict__ fstart,
                                              const float4* __restrict__ solid, const int* __restrict__ solid_cell,
-                                             const int* __restrict__ sstart, bool solids, LambdaAcc& a, int& c_n,
-                                             Lists& out) {
-    const int slab = g.gx * g.gz;
-    if (!HASHED && COMPACT) {
-        // each row's two bounds loaded just before its walk (fewer live
-        // registers than a layer's six: more resident warps)
+                                             const int* __restrict__ sstart, bool near, L& out) {
+    if constexpr (!HASHED) {
+        // 4 candidates at a time for column lists, 2 for compact ones (their
+        // build is held to 40 registers)
+        constexpr int W = CODES ? 4 : 2;
+        const int slab = g.gx * g.gz;
         const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, g.gz - 1);
+#pragma unroll 1
         for (int dy = -1; dy <= 1; dy++) {
             const int y = c.y + dy;
             if (y < 0 || y >= g.gy) continue;
+#pragma unroll 1
             for (int dx = -1; dx <= 1; dx++) {
-                const int xx = c.x + dx;
-                if (xx < 0 || xx >= g.gx) continue;
-                const int row = g.off + y * slab + xx * g.gz;
-                walk_range<MIXED, false, KAHAN, Lists, 2, PH>(p, self, s, xs, fstart[row + z0], fstart[row + z1 + 1],
-                                                              0, 0, z0 - c.z, dx, dy, a, c_n, out);
+                const int x = c.x + dx;
+                if (x < 0 || x >= g.gx) continue;
+                const int row = g.off + y * slab + x * g.gz;
+                const int i1 = row + z0 + 1, i2 = row + min(z0 + 2, z1 + 1);  // the second and third cell
+                const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) | (1 << 29) : 0;
+                walk_range<MIXED, W>(p, self, s, xs, fstart[row + z0], fstart[row + z1 + 1], MIXED ? fstart[i1] : 0,
+                                     MIXED ? fstart[i2] : 0, z0 - c.z, code, out);
+                if (SOLIDS && near)
+                    walk_range<MIXED, W>(p, self, -1, solid, sstart[row + z0], sstart[row + z1 + 1],
+                                         MIXED ? sstart[i1] : 0, MIXED ? sstart[i2] : 0, z0 - c.z,
+                                         code | (int)0x80000000u, out);
             }
         }
-    } else if (!HASHED) {
-        const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, g.gz - 1);
+    } else {
+        // cells past the packed field widths hold no particle; the dense
+        // walk's entry order: a row's fluid cells, then its solid cells
+        const int z0 = max(c.z - 1, 0), z1 = min(min(c.z + 1, g.gz - 1), (int)cp.mz);
         for (int dy = -1; dy <= 1; dy++) {
             const int y = c.y + dy;
-            if (y < 0 || y >= g.gy) continue;
-            // the fluid slot ranges of the layer's three rows, loaded together
-            int b0[3], b1[3], b2[3], b3[3];
+            if (y < 0 || y >= g.gy || y > (int)cp.my) continue;
+            for (int dx = -1; dx <= 1; dx++) {
+                const int x = c.x + dx;
+                if (x < 0 || x >= g.gx || x > (int)cp.mx) continue;
+                int a[3], b[3];
 #pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const int xx = c.x + r - 1;
-                b0[r] = b1[r] = b2[r] = b3[r] = 0;
-                if (xx >= 0 && xx < g.gx) {
-                    const int row = g.off + y * slab + xx * g.gz;
-                    b0[r] = fstart[row + z0];
-                    b3[r] = fstart[row + z1 + 1];
-                    if (MIXED) {
-                        b1[r] = fstart[row + z0 + 1];
-                        b2[r] = (z0 + 1 <= z1) ? fstart[row + z0 + 2] : b1[r];
+                for (int k = 0; k < 3; k++) {
+                    a[k] = b[k] = 0;
+                    if (z0 + k <= z1) {
+                        const int bucket = cell_bucket(make_int3(x, y, z0 + k), p.hash_bits);
+                        a[k] = fstart[bucket];
+                        b[k] = fstart[bucket + 1];
                     }
                 }
-            }
+                const int packed = (int)pack_bits(cp, make_int3(x, y, z0));
+                const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) | ((z0 - c.z + 1) << 29) : 0;
+                const int next_code = CODES ? 1 << 29 : 0;
 #pragma unroll
-            for (int r = 0; r < 3; r++) {
-                const int xx = c.x + r - 1;
-                if (xx < 0 || xx >= g.gx) continue;
-                walk_range<MIXED, false, KAHAN, Lists, COMPACT ? 2 : 4, PH>(p, self, s, xs, b0[r], b3[r], b1[r], b2[r],
-                                                                         z0 - c.z, r - 1, dy, a, c_n, out);
-                if (solids)
-                    walk_row<MIXED, true, KAHAN, Lists, PH>(p, self, s, solid, sstart, g.off + y * slab + xx * g.gz,
-                                                            c.z, g.gz, r - 1, dy, a, c_n, out);
-            }
-        }
-    }
-    for (int dy = -1; dy <= 1 && HASHED; dy++) {
-        const int y = c.y + dy;
-        if (y < 0 || y >= g.gy) continue;
-        for (int dx = -1; dx <= 1; dx++) {
-            const int xx = c.x + dx;
-            if (xx < 0 || xx >= g.gx) continue;
-            {
-                // cells past the packed field widths hold no particle
-                if (xx > (int)cp.mx || y > (int)cp.my) continue;
-                // the dense walk's entry order: the row's fluid cells, then its solid cells
-                const int z0 = max(c.z - 1, 0), z1 = min(min(c.z + 1, g.gz - 1), (int)cp.mz);
-                for (int z = z0; z <= z1; z++) {
-                    const int3 cn = make_int3(xx, y, z);
-                    walk_hashed_cell<MIXED, false, KAHAN, Lists, PH>(p, self, s, xs, fstart, cell_sorted,
-                                                                     cell_bucket(cn, p.hash_bits),
-                                                                     (int)pack_bits(cp, cn), dx, dy, z - c.z, a, c_n,
-                                                                     out);
-                }
-                if (solids)
+                for (int k = 0; k < 3; k++)
+                    walk_bucket<MIXED>(p, self, s, xs, cell_sorted, packed + (k << cp.bz_shift), a[k], b[k],
+                                       code + k * next_code, out);
+                if (SOLIDS && near)
                     for (int z = z0; z <= z1; z++) {
-                        const int3 cn = make_int3(xx, y, z);
-                        walk_hashed_cell<MIXED, true, KAHAN, Lists, PH>(p, self, s, solid, sstart, solid_cell,
-                                                                        cell_bucket(cn, p.hash_bits),
-                                                                        (int)pack_bits(cp, cn), dx, dy, z - c.z, a,
-                                                                        c_n, out);
+                        const int bucket = cell_bucket(make_int3(x, y, z), p.hash_bits);
+                        walk_bucket<MIXED>(p, self, -1, solid, solid_cell, packed + ((z - z0) << cp.bz_shift),
+                                           sstart[bucket], sstart[bucket + 1],
+                                           (code + ((z - z0) << 29)) | (int)0x80000000u, out);
                     }
             }
         }
@@ -385,24 +416,32 @@ __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack
 // FRAME: mixed storage with the iterations in the scene frame (positions
 // relative to the box corner, compensated density sums; the walk's cell is
 // the step's key, which rounding of the frame position could move).
-// FORMAT 1 or 2: compact lists (in wide records with 2) to p.rec (no cell
-// codes, no static particles).  Column lists sum the first lambda as the
-// walk accepts each candidate.  Compact lists walk first, only listing the
-// accepted candidates (no sums live across the walk: fewer registers, so
-// more resident warps), and then sum over the finished list, two entries'
-// positions loaded together (in the cache from the walk); a list cut at the
-// capacity walks once more to sum the dropped entries after the listed
-// ones.  The terms and their order are the walk's, so the sums equal the
-// column lists'.
-template <bool MIXED, bool HASHED, bool FRAME, int FORMAT>
+// FORMAT: StagedEntries (compact lists hold no static particles and no cell
+// codes).  The stencil is walked first, only listing the accepted candidates
+// (no sums live across the walk: fewer registers, so more resident warps, and
+// no pair term evaluated for the few lanes of a warp that accept), then the
+// first lambda sums over the finished list, two entries' positions loaded
+// together (in the cache from the walk); a list cut at the capacity walks once
+// more to sum the dropped entries after the listed ones, so that the terms
+// and their order do not depend on the capacity or the format.
+template <bool MIXED, bool HASHED, bool FRAME, int FORMAT, bool SOLIDS, int B>
 __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack& cp, float4* __restrict__ xs,
                                              const int* __restrict__ key_sorted, const int* __restrict__ cell_sorted,
                                              const int* __restrict__ fstart, const float4* __restrict__ solid,
                                              const int* __restrict__ solid_cell, const int* __restrict__ sstart,
                                              int* __restrict__ nbr, int* __restrict__ cnt, float* __restrict__ rho,
-                                             int* status, unsigned* stage = nullptr) {
+                                             int* status) {
+    static_assert(FORMAT == L_COLUMN || (!MIXED && !SOLIDS), "compact lists");
+    constexpr bool CODES = FORMAT == L_COLUMN;
+    using Staged = StagedEntries<FORMAT, B, FORMAT == L_COLUMN && !HASHED>;
+    __shared__ unsigned stage[Staged::WORDS];
+    // the cell shifts of the entries: from a table on a dense grid, formed per
+    // entry on a hashed one (whose walk leaves it no registers: 200 against 177 us)
+    constexpr bool TABLE = MIXED && !HASHED;
+    __shared__ float4 shift_tab[TABLE ? 64 : 1];
     pdl_wait();
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (TABLE) fill_shift_table(p, shift_tab);
+    const int s = blockIdx.x * B + threadIdx.x;
     if (s >= p.n) return;
     const float4 self = xs[s];
     const Geo g = geo_slot(p, s);
@@ -410,40 +449,38 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
     constexpr bool KAHAN = MIXED || FRAME;
     const int3 c = (MIXED || HASHED || FRAME) ? slot_cell(p, cp, g, key_sorted, cell_sorted, s)
                                               : plain_cell(p, g, self.x, self.y, self.z);
-    LambdaAcc a = lambda_init(p);
-    int c_n = 0;
-    constexpr bool COMPACT = FORMAT != 0;
-    using Lists = typename ListsOf<FORMAT>::T;
-    Lists out = open_lists((Lists*)nullptr, nbr, p.n, s, g.slot0, stage);
+    Staged out(stage, nbr, p, s, g.slot0);
     // static particles only where the cell's neighbourhood holds some
-    const bool solids = p.ns > 0 && p.solid_near && __ldg(&p.solid_near[__ldg(&key_sorted[s])]);
-    walk_stencil<COMPACT ? 1 : 0, MIXED, HASHED, KAHAN, COMPACT>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid,
-                                                                 solid_cell, sstart, solids, a, c_n, out);
-    if constexpr (COMPACT) {
-        // compact lists hold fluid slots only, with fp32 offsets: d as the walk formed it
-        const int m = min(c_n, p.max_nbrs);
-        for (int k = 0; k < m; k += 2) {
-            const bool two = k + 1 < m;
-            const float4 q0 = xs[out.get(k)];
-            const float4 q1 = two ? xs[out.get(k + 1)] : q0;
-            lambda_accumulate<KAHAN>(
-                p, a, make_float3(__fsub_rn(self.x, q0.x), __fsub_rn(self.y, q0.y), __fsub_rn(self.z, q0.z)), false);
-            if (two)
-                lambda_accumulate<KAHAN>(
-                    p, a, make_float3(__fsub_rn(self.x, q1.x), __fsub_rn(self.y, q1.y), __fsub_rn(self.z, q1.z)),
-                    false);
-        }
-        if (c_n > p.max_nbrs) {
-            int c2 = 0;
-            walk_stencil<2, MIXED, HASHED, KAHAN, COMPACT>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid,
-                                                           solid_cell, sstart, solids, a, c2, out);
-        }
+    const bool near = SOLIDS && p.ns > 0 && p.solid_near && __ldg(&p.solid_near[__ldg(&key_sorted[s])]);
+    walk_stencil<MIXED, HASHED, SOLIDS, CODES>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid, solid_cell,
+                                               sstart, near, out);
+    int c_n = out.count();
+    const int m = min(c_n, p.max_nbrs);
+    LambdaAcc a = lambda_init(p);
+    auto position = [&](int e) {
+        if (FORMAT != L_COLUMN) return xs[e];  // compact entries are slots
+        return SOLIDS ? load_entry(e, xs, solid) : xs[entry_slot(e)];
+    };
+    int solids = 0;  // the sign bit: a static particle among the entries
+    for (int k = 0; k < m; k += 2) {
+        const bool two = k + 1 < m;
+        const int e0 = out.get(p, k), e1 = two ? out.get(p, k + 1) : e0;
+        const float4 q0 = position(e0), q1 = position(e1);
+        if (SOLIDS) solids |= e0 | e1;
+        auto rel = [&](const float4& q, int e) {
+            return TABLE ? rel_t<TABLE>(self, q, e, shift_tab) : rel_entry<MIXED>(p, self, q, e);
+        };
+        lambda_accumulate<KAHAN, MIXED>(p, a, rel(q0, e0), SOLIDS && entry_solid(e0));
+        if (two) lambda_accumulate<KAHAN, MIXED>(p, a, rel(q1, e1), SOLIDS && entry_solid(e1));
     }
     if (c_n > p.max_nbrs) {
+        DroppedEntries<MIXED, KAHAN> rest{a, self, xs, solid, 0};
+        walk_stencil<MIXED, HASHED, SOLIDS, CODES>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid, solid_cell,
+                                                   sstart, near, rest);
         set_status(status, ST_NBR_OVERFLOW);
         c_n = p.max_nbrs;
     }
-    close_lists(p, out, cnt, c_n);
+    out.close(p, s, cnt, c_n, solids < 0);
     // lambda into w in place: neighbours read only xyz of this element here
     reinterpret_cast<float*>(xs)[4 * (size_t)s + 3] = lambda_of(p, a);
     if (rho) rho[s] = density_of(p, a);
@@ -459,16 +496,16 @@ __global__ void __launch_bounds__(B) k_lists_lambda(StepParams p, CellPack cp, f
                                                     const int* __restrict__ sstart,
                                                     int* __restrict__ nbr, int* __restrict__ cnt,
                                                     float* __restrict__ rho, int* status) {
-    lists_lambda<MIXED, HASHED, FRAME, 0>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell, sstart, nbr,
-                                          cnt, rho, status);
+    lists_lambda<MIXED, HASHED, FRAME, 0, true, B>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
+                                                   sstart, nbr, cnt, rho, status);
 }
 
-// Compact lists (no static particles, fp32 pair offsets; WIDE: wide records).
+// Compact lists (no static particles, fp32 pair offsets).
 // Held to 12 blocks of 128 threads per SM (40 registers, a few bytes
 // spilled): the extra resident warps hide more of the gathers' latency
 // (config 3: 0.382 -> 0.353 ms a step; a walk that loads the next row's
 // bounds ahead, or 4 gathers in flight, was slower).
-template <bool HASHED, int B, bool FRAME, bool WIDE>
+template <bool HASHED, int B, bool FRAME, int FMT>
 __global__ void __launch_bounds__(B, 1536 / B) k_lists_compact(StepParams p, CellPack cp, float4* __restrict__ xs,
                                                              const int* __restrict__ key_sorted,
                                                              const int* __restrict__ cell_sorted,
@@ -478,9 +515,8 @@ __global__ void __launch_bounds__(B, 1536 / B) k_lists_compact(StepParams p, Cel
                                                              const int* __restrict__ sstart,
                                                              int* __restrict__ nbr, int* __restrict__ cnt,
                                                              float* __restrict__ rho, int* status) {
-    __shared__ unsigned stage[COMPACT_STRIDE * B];
-    lists_lambda<false, HASHED, FRAME, WIDE ? 2 : 1>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
-                                                     sstart, nbr, cnt, rho, status, stage);
+    lists_lambda<false, HASHED, FRAME, FMT, false, B>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
+                                                      sstart, nbr, cnt, rho, status);
 }
 
 // Walk a particle's list U entries at a time, calling f(entry, position)
@@ -495,16 +531,9 @@ __global__ void __launch_bounds__(B, 1536 / B) k_lists_compact(StepParams p, Cel
 // build's pad) and the buffer holds at least LIST_PAD_MAX rows (2
 // LIST_PAD_MAX when a count exceeds LIST_PAD_MAX), so every entry a chunk
 // below the count reads is valid and every load in bounds.
-template <int U, bool SOL, int E = U, class F>
-__device__ __forceinline__ void for_each_entry(const StepParams& p, const int* __restrict__ col,
-                                               const int* __restrict__ cnt, int s,
-                                               const float4* __restrict__ xs,
-                                               const float4* __restrict__ solid, F&& f) {
-    static_assert(E % U == 0 && E <= LIST_PAD_MAX, "prefetch depth");
-    int e0[E];
-#pragma unroll
-    for (int u = 0; u < E; u++) e0[u] = __ldg(&col[(size_t)u * p.n]);
-    const int c = __ldg(&cnt[s]);
+template <int U, bool SOL, int E, class F>
+__device__ __forceinline__ void walk_column(const StepParams& p, const int* __restrict__ col, const int (&e0)[E], int c,
+                                            const float4* __restrict__ xs, const float4* __restrict__ solid, F&& f) {
     if (E > U) {
 #pragma unroll
         for (int k = 0; k < E; k += U) {
@@ -536,6 +565,24 @@ __device__ __forceinline__ void for_each_entry(const StepParams& p, const int* _
 #pragma unroll
         for (int u = 0; u < U; u++) f(e[u], q[u]);
     }
+}
+// SOL: f is called as f(entry, position, true_type or false_type), whether the
+// entry may be a static particle: warps whose lists hold none (nine in ten
+// of a block lying on voxels) run the walk without the tests.
+template <int U, bool SOL, int E = U, class F>
+__device__ __forceinline__ void for_each_entry(const StepParams& p, const int* __restrict__ col,
+                                               const int* __restrict__ cnt, int s,
+                                               const float4* __restrict__ xs,
+                                               const float4* __restrict__ solid, F&& f) {
+    static_assert(E % U == 0 && E <= LIST_PAD_MAX, "prefetch depth");
+    int e0[E];
+#pragma unroll
+    for (int u = 0; u < E; u++) e0[u] = __ldg(&col[(size_t)u * p.n]);
+    const int raw = __ldg(&cnt[s]), c = raw & ~CNT_SOLID;
+    if (SOL && __any_sync(__activemask(), raw & CNT_SOLID))
+        walk_column<U, true>(p, col, e0, c, xs, solid, [&](int e, const float4& q) { f(e, q, std::true_type()); });
+    else
+        walk_column<U, false>(p, col, e0, c, xs, solid, [&](int e, const float4& q) { f(e, q, std::false_type()); });
 }
 
 // P particles per thread: the lists of slots s[0..P) walked together, U
@@ -570,17 +617,10 @@ __device__ __forceinline__ void for_each_entry_p(const StepParams& p, const int*
     }
 }
 
-// Field j of a record: .y .z .w of the first, .x .y .z .w of the second.
-template <bool FIRST>
-__device__ __forceinline__ unsigned record_field(const uint4& r, int j) {
-    const int f = j + (FIRST ? 1 : 0);
-    return f == 0 ? r.x : (f == 1 ? r.y : (f == 2 ? r.z : r.w));
-}
-
 // The entries [K0, K0 + M) of a compact list from record r (K0 = 0: the
 // first record), min(U, M) gathers at a time; false once the count is
 // reached.
-template <int U, int M, int K0, bool WIDE, class T, class G, class F>
+template <int U, int M, int K0, int FMT, class T, class G, class F>
 __device__ __forceinline__ bool walk_record(const StepParams& p, const uint4& r, int c, int base, G&& gather,
                                             F&& f) {
     constexpr int V = U < M ? U : M;
@@ -593,12 +633,9 @@ __device__ __forceinline__ bool walk_record(const StepParams& p, const uint4& r,
 #pragma unroll
         for (int u = 0; u < V; u++)
             if (k + u < M) {
-                if (WIDE) {
-                    sl[u] = (int)record_field<K0 == 0>(r, k + u);
-                } else {
-                    const unsigned x = record_field<K0 == 0>(r, (k + u) >> 1);
-                    sl[u] = compact_slot(p, base, ((k + u) & 1) ? (x >> 16) : (x & 0xFFFFu));
-                }
+                const unsigned x = record_entry<FMT, K0 == 0>(r, k + u);
+                // one gather at a time never reads past the count
+                sl[u] = FMT != L_C16 ? (int)x : (V == 1 ? base + (int)x : compact_slot(p, base, x));
                 q[u] = gather(sl[u]);
             }
 #pragma unroll
@@ -612,19 +649,19 @@ __device__ __forceinline__ bool walk_record(const StepParams& p, const uint4& r,
 // nbr + s, its overflow rows): gather(slot) loads what f(slot, value) needs
 // of each neighbour.  A record's entries go min(U, its entries) at a time,
 // all gathers of a chunk in flight together, so with U >= 4 a list of up to
-// 4 neighbours (3 in wide records) waits for one round trip to DRAM (the
+// 4 neighbours (3 in 32-bit records) waits for one round trip to DRAM (the
 // record, with the particle's own loads) and one to L2 for the neighbours;
 // the second record is loaded only for a longer list.  Past the count an
 // entry reads the sentinel slot, whose terms are exactly zero; the overflow
 // rows are padded with it to a multiple of U (the list build's pad).
-template <int U, bool WIDE, class T, class G, class F>
+template <int U, int FMT, class T, class G, class F>
 __device__ __forceinline__ void walk_compact(const StepParams& p, const uint4& r, const uint4* __restrict__ r2,
                                              const int* __restrict__ col, G&& gather, F&& f) {
-    using RF = RecordFormat<WIDE>;
-    const int c = WIDE ? (int)r.x : (int)(r.x & 0xFFu);
-    const int base = WIDE ? 0 : (int)(r.x >> 8);
-    if (!walk_record<U, RF::INLINE, 0, WIDE, T>(p, r, c, base, gather, f)) return;
-    if (!walk_record<U, RF::EXT, RF::INLINE, WIDE, T>(p, __ldg(r2), c, base, gather, f)) return;
+    using RF = RecordFormat<FMT>;
+    const int c = FMT == L_C32 ? (int)r.x : (int)(r.x & 0xFFu);
+    const int base = FMT == L_C16 ? (int)(r.x >> 8) : 0;
+    if (!walk_record<U, RF::INLINE, 0, FMT, T>(p, r, c, base, gather, f)) return;
+    if (!walk_record<U, RF::EXT, RF::INLINE, FMT, T>(p, __ldg(r2), c, base, gather, f)) return;
     constexpr int R = RF::RECORDS;
     int nx[U];
 #pragma unroll
@@ -645,6 +682,13 @@ __device__ __forceinline__ void walk_compact(const StepParams& p, const uint4& r
     }
 }
 
+// The list format of a pass: F bit 3 compact, with bit 4 24-bit, with bit 5
+// 32-bit records.
+template <int F>
+struct ListFormatOf {
+    static constexpr int value = !(F & 8) ? L_COLUMN : ((F & 32) ? L_C32 : ((F & 16) ? L_C24 : L_C16));
+};
+
 // Lambda pass over the lists (iterations after the first); U neighbour
 // gathers in flight per thread.
 // F: bit 0 mixed precision, bit 1 the scene has static particles (the
@@ -655,9 +699,10 @@ __global__ void __launch_bounds__(B) k_lambda(StepParams p, float4* __restrict__
                                               const float4* __restrict__ solid,
                                               float* __restrict__ rho) {
     // F bit 2: the scene frame (fp32 pair offsets, compensated density sums)
-    // F bit 3: compact lists (fp32 pair offsets, no static particles); bit 4: in wide records
+    // F bits 3-5: compact lists (fp32 pair offsets, no static particles), ListFormatOf
     constexpr bool MIXED = (F & 1) != 0, SOL = (F & 2) != 0, KAHAN = MIXED || (F & 4) != 0;
-    constexpr bool COMPACT = (F & 8) != 0, WIDE = (F & 16) != 0;
+    constexpr int FMT = ListFormatOf<F>::value;
+    constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL && P == 1), "compact lists");
     pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
@@ -668,13 +713,13 @@ __global__ void __launch_bounds__(B) k_lambda(StepParams p, float4* __restrict__
         const float4 self = xs[s];
         LambdaAcc a = lambda_init(p);
         if (COMPACT) {
-            walk_compact<U, WIDE, float4>(
+            walk_compact<U, FMT, float4>(
                 p, __ldg(&p.rec[s]), p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
                 [&](int, float4 q) { lambda_accumulate<KAHAN>(p, a, rel_t<false>(self, q, 0, shift_tab), false); });
         } else {
-            for_each_entry<U, SOL>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q) {
+            for_each_entry<U, SOL>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q, auto sol) {
                 float3 d = rel_t<MIXED>(self, q, e, shift_tab);
-                lambda_accumulate<KAHAN>(p, a, d, SOL && entry_solid(e));
+                lambda_accumulate<KAHAN, MIXED>(p, a, d, decltype(sol)::value && entry_solid(e));
             });
         }
         reinterpret_cast<float*>(xs)[4 * (size_t)s + 3] = lambda_of(p, a);
@@ -689,13 +734,13 @@ __global__ void __launch_bounds__(B) k_lambda(StepParams p, float4* __restrict__
     for (int r = 0; r < P; r++) {
         s[r] = (blockIdx.x * P + r) * B + threadIdx.x;
         const bool ok = s[r] < p.n;
-        c[r] = ok ? __ldg(&cnt[s[r]]) : 0;
+        c[r] = ok ? __ldg(&cnt[s[r]]) & ~CNT_SOLID : 0;
         self[r] = ok ? xs[s[r]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         a[r] = lambda_init(p);
     }
     for_each_entry_p<U, P, SOL>(p, nbr, s, c, xs, solid, [&](int r, int e, float4 q) {
         float3 d = rel_t<MIXED>(self[r], q, e, shift_tab);
-        lambda_accumulate<KAHAN>(p, a[r], d, SOL && entry_solid(e));
+        lambda_accumulate<KAHAN, MIXED>(p, a[r], d, SOL && entry_solid(e));
     });
 #pragma unroll
     for (int r = 0; r < P; r++) {
@@ -719,7 +764,7 @@ __device__ __forceinline__ void delta_pair(const StepParams& p, DeltaAcc& a, con
     const bool sol = SOL && entry_solid(e);
     float3 d = rel_t<MIXED>(self, q, e, tab);
     const float r2 = dot3e(d.x, d.y, d.z);
-    const float inv_r = inv_r_of(r2);
+    const float inv_r = inv_r_of<MIXED>(r2);
     const float r = __fmul_rn(r2, inv_r);
     const float lj = sol ? li : q.w;
     const float w = __fmul_rn(__fadd_rn(__fadd_rn(li, lj), scorr_hd<POW>(p, hdiff(p, r2))), spiky_g(p, r, inv_r));
@@ -801,7 +846,9 @@ __global__ void __launch_bounds__(B, ((F & 8) && U == 1) ? 2048 / B : ((U <= 2 &
     k_delta(StepParams p, CellPack cp, const float4* __restrict__ xs, float4* __restrict__ xs_out,
             const int* __restrict__ nbr, const int* __restrict__ cnt, const float4* __restrict__ solid,
             const int* __restrict__ key_sorted, const float4* __restrict__ x, float4* __restrict__ v_out) {
-    constexpr bool MIXED = (F & 1) != 0, SOL = (F & 2) != 0, COMPACT = (F & 8) != 0, WIDE = (F & 16) != 0;
+    constexpr bool MIXED = (F & 1) != 0, SOL = (F & 2) != 0;
+    constexpr int FMT = ListFormatOf<F>::value;
+    constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL && P == 1), "compact lists");
     pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
@@ -811,16 +858,16 @@ __global__ void __launch_bounds__(B, ((F & 8) && U == 1) ? 2048 / B : ((U <= 2 &
         if (s >= p.n) return;
         const float4 self = xs[s];
         const uint4 rec = COMPACT ? __ldg(&p.rec[s]) : make_uint4(0u, 0u, 0u, 0u);
-        const int scene = (COMPACT && !WIDE) ? scene_of_record(p, rec.x) : scene_index(p, s);
+        const int scene = FMT == L_C16 ? scene_of_record(p, rec.x) : scene_index(p, s);
         const int packed = (MIXED && p.cell_sorted) ? __ldg(&p.cell_sorted[s]) : 0;
         DeltaAcc a{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0};
         if (COMPACT) {
-            walk_compact<U, WIDE, float4>(
+            walk_compact<U, FMT, float4>(
                 p, rec, p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
                 [&](int t, float4 q) { delta_pair<false, false, false>(p, a, self, t, q, shift_tab); });
         } else {
-            for_each_entry<U, SOL, LIST_PAD_MAX>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q) {
-                delta_pair<MIXED, SOL>(p, a, self, e, q, shift_tab);
+            for_each_entry<U, SOL, LIST_PAD_MAX>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q, auto sol) {
+                delta_pair<MIXED, decltype(sol)::value>(p, a, self, e, q, shift_tab);
             });
         }
         delta_finish<MIXED>(p, cp, s, self, a, xs_out, key_sorted, x, v_out, scene, packed);
@@ -833,7 +880,7 @@ __global__ void __launch_bounds__(B, ((F & 8) && U == 1) ? 2048 / B : ((U <= 2 &
     for (int r = 0; r < P; r++) {
         s[r] = (blockIdx.x * P + r) * B + threadIdx.x;
         const bool ok = s[r] < p.n;
-        c[r] = ok ? __ldg(&cnt[s[r]]) : 0;
+        c[r] = ok ? __ldg(&cnt[s[r]]) & ~CNT_SOLID : 0;
         self[r] = ok ? xs[s[r]] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         a[r] = DeltaAcc{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0};
     }
@@ -877,7 +924,9 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
                                             float4* __restrict__ xs_next, int* __restrict__ key,
                                             int* __restrict__ rank, int* __restrict__ count, int* __restrict__ cellk,
                                             int* __restrict__ tile_count) {
-    constexpr bool MIXED = (F & 1) != 0, SOL = (F & 2) != 0, COMPACT = (F & 8) != 0, WIDE = (F & 16) != 0;
+    constexpr bool MIXED = (F & 1) != 0, SOL = (F & 2) != 0;
+    constexpr int FMT = ListFormatOf<F>::value;
+    constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL), "compact lists");
     pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
@@ -897,11 +946,11 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     const int* __restrict__ col = nbr + s;
     float ax = 0.0f, ay = 0.0f, az = 0.0f;
     if (COMPACT && p.c_xsph != 0.0f) {
-        walk_compact<U, WIDE, PosVel>(
+        walk_compact<U, FMT, PosVel>(
             p, rec, p.rec2 + s, col, [&](int t) { return PosVel{xs[t], v_in[t]}; },
             [&](int t, const PosVel& q) { xsph_pair<false>(p, self, vi, q.x, q.v, t, shift_tab, ax, ay, az); });
     } else if (p.c_xsph != 0.0f) {
-        const int c = cnt[s];
+        const int c = cnt[s] & ~CNT_SOLID;
         const int sent = sentinel_entry(p);
         for (int k = 0; k < c; k += U) {
             int e[U];
@@ -924,7 +973,7 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     const float cx = __fmul_rn(p.c_xsph, p.k6);
     const float4 vc = make_float4(__fmaf_rn(cx, ax, vi.x), __fmaf_rn(cx, ay, vi.y), __fmaf_rn(cx, az, vi.z), 0.0f);
     v_out[s] = vc;
-    const Geo g = (COMPACT && !WIDE) ? geo_of(p, scene_of_record(p, rec.x))
+    const Geo g = FMT == L_C16 ? geo_of(p, scene_of_record(p, rec.x))
                                      : geo_slot(p, s);
     float4 xc;
     if (!MIXED && !p.frame) {

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(T, 1) k_scene_solve(StepParams p, CellPack cp,
                     const float3 d = make_float3(__fsub_rn(self.x, q.x), __fsub_rn(self.y, q.y),
                                                  __fsub_rn(self.z, q.z));
                     const float r2 = dot3e(d.x, d.y, d.z);
-                    const float inv_r = inv_r_of(r2);
+                    const float inv_r = inv_r_of<false>(r2);
                     const float r = __fmul_rn(r2, inv_r);
                     const float w = __fmul_rn(__fadd_rn(__fadd_rn(li, q.w), scorr_hd(p, hdiff(p, r2))),
                                               spiky_g(p, r, inv_r));
