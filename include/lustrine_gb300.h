@@ -451,7 +451,9 @@ LUSTRINE_API int lustrine_pbf_profile_step(lustrine_pbf* s, float dt, double* st
  * thread: 16-bit entries for scenes of at most
  * 65,535 in contexts of fewer than 2^24 fluid particles, wide records
  * otherwise; elsewhere the step keeps column lists whatever list_format
- * says). */
+ * says).  Until a shape is set or autotuned, get_tuning reports the library's
+ * default, and the step itself picks the gathers in flight by list format and
+ * particle count (the results are the same bits in every shape). */
 enum {
     LUSTRINE_LISTS_COLUMN = 0,       /* count + column-major 32-bit entries */
     LUSTRINE_LISTS_COMPACT = 1,      /* 16-byte records: count, scene's first slot, 6 (+8) 16-bit offsets */

@@ -272,6 +272,38 @@ static int compact_now(const lustrine_pbf* s) {
     return compact_capable(s);
 }
 
+// The launch shape of a step's passes: the one that was set or autotuned, else
+// by list format and size.  More gathers in flight shorten a particle's chain of
+// dependent loads but take registers (U = 4: 56, nine blocks of 128 per SM), so
+// they pay while all particles still fit the GPU at once, ONE_WAVE of them.
+// Measured, us per step at the fixed shape (2 gathers, 8 in XSPH) and at this
+// rule's, 4 iterations:
+//   column lists, fp32 with static particles: 77,000 63.7 / 58.8, 150,000
+//     87.7 / 74.3, 262,144 99.6 / 94.8, 500,000 155 / 153
+//   column lists, per-cell mixed: 150,000 94.8 / 88.0 with 4 and 4 (2 and 2:
+//     93.7), 300,000 128 / 126 with 2 and 2 (4 and 4: 132), 3 M hashed 1141 / 1119
+//   16-bit records: 10,000 37.1 / 35.5, 37 scenes of 157,443 73.4 / 69.9;
+//     200 scenes of 3.0 M 573 / 545 with 1 and 4 (4 and 4: 576)
+//   24-bit records: 200,000 62.1 (2 and 2: 63.2), 600,000 162.5 / 161.8,
+//     2 M 497 / 492 (4 and 4: 522)
+constexpr int ONE_WAVE = 152 * 9 * 128;
+constexpr int XSPH_WIDE_MAX = 250000;
+static Tuning launch_shape(const lustrine_pbf* s, int format) {
+    Tuning t = s->tune;
+    if (s->tune_set) return t;
+    const bool small = s->n <= ONE_WAVE;
+    if (format == LUSTRINE_LISTS_COMPACT_WIDE) {
+        t.xsph_unroll = s->n <= XSPH_WIDE_MAX ? 8 : 2;
+    } else if (format == LUSTRINE_LISTS_COMPACT) {
+        t.unroll = small ? 4 : 1;
+        t.xsph_unroll = 4;
+    } else {
+        const bool cells = s->mixed() && !s->sp.frame;
+        t.unroll = t.xsph_unroll = cells && !small ? 2 : 4;
+    }
+    return t;
+}
+
 // Device buffers for s->cap fluid particles (s->n of them active).
 static int ctx_alloc(lustrine_pbf* s) {
     const int n = s->cap, ns = s->ns, C = s->sp.num_cells, m = n > ns ? n : ns;
@@ -1015,7 +1047,7 @@ static int enqueue_step(lustrine_pbf* s, cudaStream_t st, StageMarks* mk = nullp
         float4* a = s->xs[o];
         float4* b = s->xs_alt;
         const int iters = s->prm.iterations;
-        const Tuning& tu = s->tune;
+        const Tuning tu = launch_shape(s, s->lists_format);
         for (int it = 0; it < iters; it++) {
             float* rho = it == iters - 1 ? s->rho : nullptr;  // densities of the last pass only
             if (it == 0) {
@@ -1212,6 +1244,7 @@ extern "C" int lustrine_pbf_set_tuning(lustrine_pbf* s, const lustrine_pbf_tunin
         return LUSTRINE_ERR_ARGS;
     }
     s->tune = Tuning{t->block, t->unroll, t->list_block, xu, ppt, t->list_format};
+    s->tune_set = true;
     s->invalidate_graphs();
     return LUSTRINE_OK;
 }
@@ -1312,6 +1345,8 @@ extern "C" int lustrine_pbf_autotune(lustrine_pbf* s, float dt, int steps, lustr
     int rc = snapshot_take(s, sn);
     const int side = s->cur;
     Tuning keep = s->tune, top = s->tune;
+    const bool keep_set = s->tune_set;
+    s->tune_set = true;
     const bool keep_onchip = s->onchip;
     const int keep_threads = s->onchip_threads;
     s->onchip = false;  // the per-stage kernels' shapes first
@@ -1380,6 +1415,7 @@ extern "C" int lustrine_pbf_autotune(lustrine_pbf* s, float dt, int steps, lustr
         }
     }
     s->tune = rc ? keep : top;
+    s->tune_set = rc ? keep_set : true;
     s->onchip = rc ? keep_onchip : top_onchip;
     s->onchip_threads = rc ? keep_threads : top_threads;
     s->invalidate_graphs();

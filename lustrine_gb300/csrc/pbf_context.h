@@ -23,6 +23,7 @@ struct lustrine_pbf {
     lgb::StepParams sp{};
     lgb::CellPack cp{};
     lgb::Tuning tune{128, 2, 128, 8, 1, 1};
+    bool tune_set = false;  // by set_tuning or the autotuner; else the step picks the passes' shape
     int n = 0, ns = 0;
     int cap = 0;  // fluid particles the buffers hold (n <= cap; sources append up to it)
     cudaStream_t stream = nullptr;
