@@ -114,6 +114,7 @@ struct StepParams {
     int frame;            // mixed storage, iterations in the scene frame (LUSTRINE_PRECISION_MIXED_SCENE)
     uint4* rec;           // compact neighbour lists of this step (nullptr: column lists with counts)
     uint4* rec2;          // their second records
+    int early;            // the lists are older than the pass's predecessor (ListHead)
     int wide;             // compact lists in wide records: 1 24-bit slots, 2 32-bit slots (0: 16-bit offsets)
     const int* src;       // the previous slot of each sorted slot, whose committed position the last
                           // position pass reads from the unsorted state (nullptr: sorted with the step)

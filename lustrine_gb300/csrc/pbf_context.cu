@@ -1058,6 +1058,7 @@ static int enqueue_step(lustrine_pbf* s, cudaStream_t st, StageMarks* mk = nullp
                 launch_lambda(mixed, tu, pl, a, s->nbr, s->cnt, s->solid, rho, st);
                 if (mk) mk->mark(LUSTRINE_STAGE_LAMBDA, st);
             }
+            pl.early = it > 0;
             launch_delta(mixed, tu, pl, s->cp, a, b, s->nbr, s->cnt, s->solid, s->key_sorted, s->x[c],
                          it == iters - 1 ? s->vtmp : nullptr, st);
             if (mk) mk->mark(LUSTRINE_STAGE_DELTA, st);

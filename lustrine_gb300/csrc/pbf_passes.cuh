@@ -569,21 +569,42 @@ __device__ __forceinline__ void walk_column(const StepParams& p, const int* __re
 // SOL: f is called as f(entry, position, true_type or false_type), whether the
 // entry may be a static particle: warps whose lists hold none (nine in ten
 // of a block lying on voxels) run the walk without the tests.
-template <int U, bool SOL, int E = U, class F>
-__device__ __forceinline__ void for_each_entry(const StepParams& p, const int* __restrict__ col,
-                                               const int* __restrict__ cnt, int s,
-                                               const float4* __restrict__ xs,
+template <int U, bool SOL, int E, class F>
+__device__ __forceinline__ void for_each_entry(const StepParams& p, const int* __restrict__ col, const int (&e0)[E],
+                                               int raw, const float4* __restrict__ xs,
                                                const float4* __restrict__ solid, F&& f) {
     static_assert(E % U == 0 && E <= LIST_PAD_MAX, "prefetch depth");
-    int e0[E];
-#pragma unroll
-    for (int u = 0; u < E; u++) e0[u] = __ldg(&col[(size_t)u * p.n]);
-    const int raw = __ldg(&cnt[s]), c = raw & ~CNT_SOLID;
+    const int c = raw & ~CNT_SOLID;
     if (SOL && __any_sync(__activemask(), raw & CNT_SOLID))
         walk_column<U, true>(p, col, e0, c, xs, solid, [&](int e, const float4& q) { f(e, q, std::true_type()); });
     else
         walk_column<U, false>(p, col, e0, c, xs, solid, [&](int e, const float4& q) { f(e, q, std::false_type()); });
 }
+
+// The start of a particle's list: its record, or its count and first E column
+// entries.  The lists are older than the pass's predecessor in the stream
+// (list build, position pass, lambda pass, position pass, ...), so a pass
+// launched behind it loads them before it waits for it: when its blocks start,
+// every block of the predecessor has passed its own wait, so whatever ran before
+// that has completed.  (The first position pass follows the list build: it
+// waits first, StepParams::early unset.)  One dependent load less a pass where
+// launches and latency count: host frames of 77,777 particles 420 -> 397 us for
+// four, 157,443 in 37 scenes 382 -> 371 for four steps; 2 M: no change.
+template <int FMT, int E>
+struct ListHead {
+    uint4 rec;
+    int raw, e0[E];
+    __device__ __forceinline__ void load(const StepParams& p, const int* __restrict__ nbr,
+                                         const int* __restrict__ cnt, int s) {
+        if (FMT != L_COLUMN) {
+            rec = __ldg(&p.rec[s]);
+        } else {
+#pragma unroll
+            for (int u = 0; u < E; u++) e0[u] = __ldg(&nbr[(size_t)u * p.n + s]);
+            raw = __ldg(&cnt[s]);
+        }
+    }
+};
 
 // P particles per thread: the lists of slots s[0..P) walked together, U
 // entries of each per round, so the loads of all P lists and their gathers
@@ -704,20 +725,23 @@ __global__ void __launch_bounds__(B) k_lambda(StepParams p, float4* __restrict__
     constexpr int FMT = ListFormatOf<F>::value;
     constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL && P == 1), "compact lists");
-    pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
-    if (MIXED) fill_shift_table(p, shift_tab);
     if (P == 1) {
-        const int s = blockIdx.x * blockDim.x + threadIdx.x;
-        if (s >= p.n) return;
+        const int s = blockIdx.x * B + threadIdx.x;
+        const bool live = s < p.n;
+        ListHead<FMT, U> head;
+        if (live) head.load(p, nbr, cnt, s);
+        pdl_wait();
+        if (MIXED) fill_shift_table(p, shift_tab);
+        if (!live) return;
         const float4 self = xs[s];
         LambdaAcc a = lambda_init(p);
         if (COMPACT) {
             walk_compact<U, FMT, float4>(
-                p, __ldg(&p.rec[s]), p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
+                p, head.rec, p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
                 [&](int, float4 q) { lambda_accumulate<KAHAN>(p, a, rel_t<false>(self, q, 0, shift_tab), false); });
         } else {
-            for_each_entry<U, SOL>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q, auto sol) {
+            for_each_entry<U, SOL>(p, nbr + s, head.e0, head.raw, xs, solid, [&](int e, float4 q, auto sol) {
                 float3 d = rel_t<MIXED>(self, q, e, shift_tab);
                 lambda_accumulate<KAHAN, MIXED>(p, a, d, decltype(sol)::value && entry_solid(e));
             });
@@ -726,6 +750,8 @@ __global__ void __launch_bounds__(B) k_lambda(StepParams p, float4* __restrict__
         if (rho) rho[s] = density_of(p, a);
         return;
     }
+    pdl_wait();
+    if (MIXED) fill_shift_table(p, shift_tab);
     // P slots per thread, B apart (each load of the block coalesced)
     int s[P], c[P];
     float4 self[P];
@@ -850,29 +876,34 @@ __global__ void __launch_bounds__(B, ((F & 8) && U == 1) ? 2048 / B : ((U <= 2 &
     constexpr int FMT = ListFormatOf<F>::value;
     constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL && P == 1), "compact lists");
-    pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
-    if (MIXED) fill_shift_table(p, shift_tab);
     if (P == 1) {
-        const int s = blockIdx.x * blockDim.x + threadIdx.x;
-        if (s >= p.n) return;
+        const int s = blockIdx.x * B + threadIdx.x;
+        const bool live = s < p.n;
+        ListHead<FMT, LIST_PAD_MAX> head;
+        if (live && p.early) head.load(p, nbr, cnt, s);
+        pdl_wait();
+        if (MIXED) fill_shift_table(p, shift_tab);
+        if (!live) return;
+        if (!p.early) head.load(p, nbr, cnt, s);
         const float4 self = xs[s];
-        const uint4 rec = COMPACT ? __ldg(&p.rec[s]) : make_uint4(0u, 0u, 0u, 0u);
-        const int scene = FMT == L_C16 ? scene_of_record(p, rec.x) : scene_index(p, s);
+        const int scene = FMT == L_C16 ? scene_of_record(p, head.rec.x) : scene_index(p, s);
         const int packed = (MIXED && p.cell_sorted) ? __ldg(&p.cell_sorted[s]) : 0;
         DeltaAcc a{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0};
         if (COMPACT) {
             walk_compact<U, FMT, float4>(
-                p, rec, p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
+                p, head.rec, p.rec2 + s, nbr + s, [&](int t) { return xs[t]; },
                 [&](int t, float4 q) { delta_pair<false, false, false>(p, a, self, t, q, shift_tab); });
         } else {
-            for_each_entry<U, SOL, LIST_PAD_MAX>(p, nbr + s, cnt, s, xs, solid, [&](int e, float4 q, auto sol) {
+            for_each_entry<U, SOL>(p, nbr + s, head.e0, head.raw, xs, solid, [&](int e, float4 q, auto sol) {
                 delta_pair<MIXED, decltype(sol)::value>(p, a, self, e, q, shift_tab);
             });
         }
         delta_finish<MIXED>(p, cp, s, self, a, xs_out, key_sorted, x, v_out, scene, packed);
         return;
     }
+    pdl_wait();
+    if (MIXED) fill_shift_table(p, shift_tab);
     int s[P], c[P];
     float4 self[P];
     DeltaAcc a[P];
@@ -928,16 +959,22 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
     constexpr int FMT = ListFormatOf<F>::value;
     constexpr bool COMPACT = FMT != L_COLUMN;
     static_assert(!COMPACT || (!MIXED && !SOL), "compact lists");
-    pdl_wait();
     __shared__ float4 shift_tab[MIXED ? 64 : 1];
     __shared__ TileSum tiles;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = s < p.n;
-    const float4 self = xs[live ? s : 0];  // in flight across the barrier
-    const float4 vi = v_in[live ? s : 0];
-    const uint4 rec = COMPACT ? __ldg(&p.rec[live ? s : 0]) : make_uint4(0u, 0u, 0u, 0u);
+    // older than the last position pass (ListHead): loaded before the wait for
+    // it, but where the 32-register kernel would spill for it
+    constexpr bool AHEAD = !(FMT == L_C24 && U == 1);
+    uint4 rec = make_uint4(0u, 0u, 0u, 0u);
+    if (COMPACT && AHEAD) rec = __ldg(&p.rec[live ? s : 0]);
+    const int raw = COMPACT ? 0 : __ldg(&cnt[live ? s : 0]);
     // the block's tile: that of its first particle's cell in this step
     if (xs_next && threadIdx.x == 0) open_tile_sum(tiles, __ldg(&key_sorted[s]));
+    pdl_wait();
+    const float4 self = xs[live ? s : 0];  // in flight across the barrier
+    const float4 vi = v_in[live ? s : 0];
+    if (COMPACT && !AHEAD) rec = __ldg(&p.rec[live ? s : 0]);
     if (MIXED)
         fill_shift_table(p, shift_tab);
     else if (xs_next)
@@ -950,7 +987,7 @@ __device__ __forceinline__ void xsph_commit(const StepParams& p, const CellPack&
             p, rec, p.rec2 + s, col, [&](int t) { return PosVel{xs[t], v_in[t]}; },
             [&](int t, const PosVel& q) { xsph_pair<false>(p, self, vi, q.x, q.v, t, shift_tab, ax, ay, az); });
     } else if (p.c_xsph != 0.0f) {
-        const int c = cnt[s] & ~CNT_SOLID;
+        const int c = raw & ~CNT_SOLID;
         const int sent = sentinel_entry(p);
         for (int k = 0; k < c; k += U) {
             int e[U];

@@ -233,9 +233,12 @@ __global__ void __launch_bounds__(CELL_SCAN_THREADS) k_scan_tiles(int* __restric
 
 __global__ void k_scatter_index(const int* __restrict__ key, const int* __restrict__ rank,
                                 const int* __restrict__ start, int n, int* __restrict__ tmp) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    // the prediction's, older than the scan before this kernel: in flight
+    // while it drains
+    const int k = i < n ? key[i] : 0, r = i < n ? rank[i] : 0;
     pdl_wait();
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) tmp[start[key[i]] + rank[i]] = i;
+    if (i < n) tmp[start[k] + r] = i;
 }
 
 // ------------------------------------------------------- stabilisation --
