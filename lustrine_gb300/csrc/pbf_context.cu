@@ -212,7 +212,7 @@ void lustrine_pbf::free_buffers() {
         host_graph[k] = nullptr;
     }
     void* ptrs[] = {x[0], x[1], xs[0], xs[1], v[0], v[1], id[0], id[1], xs_alt, xs_pred, vtmp, key, key_sorted,
-                    rank, tmp, perm, count, start, block_sums, tile_sum, solid_near, solid, solid_raw, sstart, nbr, cnt, lam,
+                    rank, tmp, perm, count, start, block_sums, solid_near, solid, solid_raw, sstart, nbr, cnt, lam,
                     lam_by_id, rho, status, red, qcount, out3, out3d, iota, slot_of, solid_id, d_scenes, d_scene_of,
                     d_solid_scene_of, cellk, cell_sorted, solid_cell, att[0], att[1], d_bins, d_scene_slot0,
                     d_queue, rec, rec2, src};
@@ -323,10 +323,12 @@ static int ctx_alloc(lustrine_pbf* s) {
     rc = rc ? rc : dalloc(&s->rank, m);
     rc = rc ? rc : dalloc(&s->tmp, m);
     rc = rc ? rc : dalloc(&s->perm, m);
-    rc = rc ? rc : dalloc(&s->count, C);
+    // the histogram, and behind it the scan's tile totals: cleared together
+    const size_t tiles_at = ((size_t)C + 31) / 32 * 32;
+    rc = rc ? rc : dalloc(&s->count, tiles_at + 2 * (size_t)cell_scan_tiles(C));
+    s->tile_sum = s->count ? s->count + tiles_at : nullptr;
     rc = rc ? rc : dalloc(&s->start, (size_t)C + 1);
     rc = rc ? rc : dalloc(&s->block_sums, scan_block_sums_size(C));
-    rc = rc ? rc : dalloc(&s->tile_sum, 2 * (size_t)cell_scan_tiles(C));
     rc = rc ? rc : dalloc(&s->solid, (size_t)ns + SPAN_PAD);
     rc = rc ? rc : dalloc(&s->solid_raw, ns);
     rc = rc ? rc : dalloc(&s->sstart, (size_t)C + 1);
@@ -713,10 +715,14 @@ static int* tiles_of(lustrine_pbf* s, int parity) {
     return s->tile_sum + (size_t)parity * cell_scan_tiles(s->sp.num_cells);
 }
 
-// Zero both halves of the tile totals (after a prediction was dropped).
-static int clear_tiles(lustrine_pbf* s) {
-    CK(cudaMemsetAsync(s->tile_sum, 0, 2 * (size_t)cell_scan_tiles(s->sp.num_cells) * sizeof(int), s->stream));
-    s->tiles_dirty = false;
+// Zero what a dropped prediction counted: the histogram where it holds one, and
+// both halves of the tile totals behind it.
+static int clear_prediction(lustrine_pbf* s) {
+    int* const from = s->count_dirty ? s->count : s->tile_sum;
+    int* const end = s->tile_sum + 2 * (size_t)cell_scan_tiles(s->sp.num_cells);
+    if (s->count_dirty || s->tiles_dirty)
+        CK(cudaMemsetAsync(from, 0, (size_t)(end - from) * sizeof(int), s->stream));
+    s->count_dirty = s->tiles_dirty = false;
     return LUSTRINE_OK;
 }
 
@@ -835,8 +841,22 @@ extern "C" int lustrine_pbf_upload_state_async(lustrine_pbf* s, const float* x, 
     if (!n) return LUSTRINE_OK;
     const float* hx = (const float*)host_view(x);
     const float* hv = (const float*)host_view(v);
-    if (hx && !s->is_batch() && (!v || hv)) {  // read straight from the page-locked buffers
+    if (hx && (!v || hv)) {  // read straight from the page-locked buffers
         const int c = s->cur;
+        if (s->prm.mode == LUSTRINE_MODE_PBF && s->sp.dt > 0.0f) {
+            // with the next step's prediction for the last step's dt: the
+            // transfer is bound by the host link, and a step with that dt then
+            // starts at its sort (another dt predicts anew).  2 M particles:
+            // the prediction kernel's 25 us.
+            int rc = clear_prediction(s);
+            if (rc) return rc;
+            launch_pack_predict(s->mixed(), s->sp, s->cp, hx, hv, n, s->x[c], s->v[c], s->id[c], s->xs_pred, s->key,
+                                s->rank, s->count, s->cellk, tiles_of(s, c), s->stream);
+            CK(cudaGetLastError());
+            s->count_dirty = s->pred_ready = true;
+            s->pred_dt = s->sp.dt;
+            return LUSTRINE_OK;
+        }
         launch_pack_state(s->mixed(), s->sp, s->cp, hx, hv, n, s->x[c], s->v[c], s->id[c], s->stream);
         CK(cudaGetLastError());
         return LUSTRINE_OK;
@@ -1133,10 +1153,8 @@ static int step_impl(lustrine_pbf* s, float dt, bool tail_allowed) {
     // the previous step predicted this one unless something changed since
     const bool predict = !(pbf && s->pred_ready && s->pred_dt == dt);
     const bool tail = pbf && tail_allowed;
-    if (predict && s->count_dirty)  // a histogram of a prediction that will not be used
-        CK(cudaMemsetAsync(s->count, 0, (size_t)s->sp.num_cells * sizeof(int), s->stream));
-    if (predict && (s->count_dirty || s->tiles_dirty)) {  // and its tile totals
-        int rc = clear_tiles(s);
+    if (predict) {  // the counts of a prediction that will not be used
+        int rc = clear_prediction(s);
         if (rc) return rc;
     }
     s->count_dirty = false;
@@ -1193,10 +1211,9 @@ extern "C" int lustrine_pbf_profile_step(lustrine_pbf* s, float dt, double* stag
         s->sp.inv_dt = 1.0f / dt;
         s->invalidate_graphs();
     }
-    if (s->count_dirty) CK(cudaMemsetAsync(s->count, 0, (size_t)s->sp.num_cells * sizeof(int), s->stream));
-    s->count_dirty = false;
     s->pred_ready = false;
-    int trc = clear_tiles(s);
+    s->tiles_dirty = true;
+    int trc = clear_prediction(s);
     if (trc) return trc;
     StageMarks mk;
     for (int e = 0; e < 64; e++) CK(cudaEventCreate(&mk.ev[e]));
@@ -1515,12 +1532,8 @@ extern "C" int lustrine_pbf_step_host(lustrine_pbf* s, float dt, float* x, float
             s->sp.inv_dt = 1.0f / dt;
             s->invalidate_graphs();
         }
-        if (s->count_dirty) CK(cudaMemsetAsync(s->count, 0, (size_t)s->sp.num_cells * sizeof(int), s->stream));
-        if (s->count_dirty || s->tiles_dirty) {
-            int rc = clear_tiles(s);
-            if (rc) return rc;
-        }
-        s->count_dirty = false;
+        int crc = clear_prediction(s);
+        if (crc) return crc;
         const int c = s->cur;
         if (!s->mixed() && s->prm.use_graph) {
             // the whole frame as one graph for this buffer pair: upload fused
@@ -1536,7 +1549,7 @@ extern "C" int lustrine_pbf_step_host(lustrine_pbf* s, float dt, float* x, float
                 s->host_graph[c] = nullptr;
                 cudaGraph_t g = nullptr;
                 CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-                launch_pack_predict(false, s->sp, s->cp, hx, hv, s->n, s->x[c], s->id[c], s->xs_pred, s->key,
+                launch_pack_predict(false, s->sp, s->cp, hx, hv, s->n, s->x[c], nullptr, s->id[c], s->xs_pred, s->key,
                                     s->rank, s->count, s->cellk, tiles_of(s, c), s->stream);
                 const HostFrame hf{const_cast<float*>(hx), const_cast<float*>(hv)};
                 const int k = 1 + enqueue_step(s, s->stream, nullptr, false, false, &hf);
@@ -1558,7 +1571,7 @@ extern "C" int lustrine_pbf_step_host(lustrine_pbf* s, float dt, float* x, float
             CK(cudaStreamSynchronize(s->stream));
             return LUSTRINE_OK;
         }
-        launch_pack_predict(s->mixed(), s->sp, s->cp, hx, hv, s->n, s->x[c], s->id[c], s->xs_pred, s->key, s->rank,
+        launch_pack_predict(s->mixed(), s->sp, s->cp, hx, hv, s->n, s->x[c], nullptr, s->id[c], s->xs_pred, s->key, s->rank,
                             s->count, s->cellk, tiles_of(s, c), s->stream);
         CK(cudaGetLastError());
         s->pred_ready = true;

@@ -161,9 +161,10 @@ void launch_pack_state(bool mixed, const StepParams& p, const CellPack& cp, cons
 void launch_unpack_state(bool mixed, const StepParams& p, const CellPack& cp, const float4* x, const float4* v,
                          const int* id, int* slot_of, bool slot_of_valid, int n, float* hx, float* hv,
                          cudaStream_t st);
-// a host frame's upload fused with the step's prediction (slot = caller index)
+// upload fused with the step's prediction (slot = caller index); v_out may be
+// nullptr (a host frame, whose step recomputes the velocities)
 void launch_pack_predict(bool mixed, const StepParams& p, const CellPack& cp, const float* hx, const float* hv,
-                         int n, float4* x, int* id, float4* xs, int* key, int* rank, int* count, int* cellk,
+                         int n, float4* x, float4* v_out, int* id, float4* xs, int* key, int* rank, int* count, int* cellk,
                          int* tile_count, cudaStream_t st);
 void launch_reduce(bool mixed, const StepParams& p, const CellPack& cp, const float4* x,
                    const float4* v, const float* rho, double* out, cudaStream_t st);

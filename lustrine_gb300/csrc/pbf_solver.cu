@@ -141,19 +141,20 @@ __global__ void __launch_bounds__(HOST_BLOCK) k_pack_state(StepParams p, CellPac
     const int i = blockIdx.x * HOST_BLOCK + threadIdx.x;
     if (i >= n) return;
     const int t = 3 * threadIdx.x;
-    x[i] = pack_position<MIXED>(p, cp, geo_single(p), sx[t], sx[t + 1], sx[t + 2]);
+    x[i] = pack_position<MIXED>(p, cp, geo_slot(p, i), sx[t], sx[t + 1], sx[t + 2]);
     v[i] = hv ? make_float4(sv[t], sv[t + 1], sv[t + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     id[i] = i;
 }
 
-// Upload fused with the step's prediction (a host frame: the state comes in
-// from page-locked memory and is stepped at once): slot = caller index, x
-// packed into the state, v used by the prediction only (the step recomputes
-// it), then predict_one as k_predict does on the same values.
+// Upload fused with the step's prediction: slot = caller index, x packed into
+// the state, and v where v_out is given (a host frame, stepped at once, has no
+// use for it: the step recomputes it), then predict_one as k_predict does on
+// the same values.
 template <bool MIXED>
 __global__ void __launch_bounds__(HOST_BLOCK) k_pack_predict(StepParams p, CellPack cp, const float* __restrict__ hx,
                                                              const float* __restrict__ hv, int n,
-                                                             float4* __restrict__ x, int* __restrict__ id,
+                                                             float4* __restrict__ x, float4* __restrict__ v_out,
+                                                             int* __restrict__ id,
                                                              float4* __restrict__ xs, int* __restrict__ key,
                                                              int* __restrict__ rank, int* __restrict__ count,
                                                              int* __restrict__ cellk, int* __restrict__ tile_count) {
@@ -167,10 +168,11 @@ __global__ void __launch_bounds__(HOST_BLOCK) k_pack_predict(StepParams p, CellP
     int k = 0;
     if (live) {
         const int t = 3 * threadIdx.x;
-        const Geo g = geo_single(p);
+        const Geo g = geo_slot(p, i);
         const float4 xi = pack_position<MIXED>(p, cp, g, sx[t], sx[t + 1], sx[t + 2]);
         const float4 vi = hv ? make_float4(sv[t], sv[t + 1], sv[t + 2], 0.0f) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         x[i] = xi;
+        if (v_out) v_out[i] = vi;
         id[i] = i;
         k = predict_one<MIXED>(p, cp, g, xi, vi, i, xs, key, rank, count, cellk);
     }
@@ -497,10 +499,10 @@ void launch_pack_state(bool mixed, const StepParams& p, const CellPack& cp, cons
 }
 
 void launch_pack_predict(bool mixed, const StepParams& p, const CellPack& cp, const float* hx, const float* hv,
-                         int n, float4* x, int* id, float4* xs, int* key, int* rank, int* count, int* cellk,
-                         int* tile_count, cudaStream_t st) {
+                         int n, float4* x, float4* v_out, int* id, float4* xs, int* key, int* rank, int* count,
+                         int* cellk, int* tile_count, cudaStream_t st) {
     if (n <= 0) return;
-    LGB_DISPATCH(mixed, k_pack_predict, blocks_for(n, HOST_BLOCK), HOST_BLOCK, st, p, cp, hx, hv, n, x, id, xs,
+    LGB_DISPATCH(mixed, k_pack_predict, blocks_for(n, HOST_BLOCK), HOST_BLOCK, st, p, cp, hx, hv, n, x, v_out, id, xs,
                  key, rank, count, cellk, tile_count);
 }
 
