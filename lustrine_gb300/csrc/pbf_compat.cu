@@ -133,9 +133,11 @@ __global__ void k_key_ref(StepParams p, const float4* __restrict__ pos, int m, i
 // cell).  Each row's bounds are loaded while the one before is walked.  Bound by
 // instruction issue at the few warps a scene of this mode has (100,000
 // particles, h = 1.55: 36.2 us cell by cell with a store to the list's row per
-// accepted candidate, 19.5 us like this).
+// accepted candidate, 19.5 us like this).  G lanes share a particle's rows where
+// a scene has few (as the sand lists do).
 constexpr int REF_BLOCK = 128;
 constexpr int REF_STAGE = 24;  // list entries staged in shared memory
+template <int G>
 __global__ void __launch_bounds__(REF_BLOCK) k_lists_ref(StepParams p, const float4* __restrict__ xs,
                                                          const int* __restrict__ key,
                                                          const int* __restrict__ fstart,
@@ -143,8 +145,9 @@ __global__ void __launch_bounds__(REF_BLOCK) k_lists_ref(StepParams p, const flo
                                                          const int* __restrict__ sstart, int* __restrict__ nbr,
                                                          int* __restrict__ cnt, int* status) {
     pdl_wait();
-    __shared__ int stage[REF_STAGE * REF_BLOCK];
-    const int s = blockIdx.x * REF_BLOCK + threadIdx.x;
+    constexpr int STAGE = G == 1 ? REF_STAGE : 12;
+    __shared__ int stage[STAGE * REF_BLOCK];
+    const int s = (blockIdx.x * REF_BLOCK + threadIdx.x) / G, g = threadIdx.x % G;
     if (s >= p.n) return;
     const float4 self = xs[s];
     const int id = key[s];
@@ -152,50 +155,60 @@ __global__ void __launch_bounds__(REF_BLOCK) k_lists_ref(StepParams p, const flo
     const int yy = id / slab, xx = (id % slab) / p.gz, zz = id % p.gz;
     const int z0 = max(zz - 1, 0), z1 = min(zz + 1, p.gz - 1);
     const bool near = p.ns > 0 && p.solid_near[id];
-    StagedList<REF_STAGE, REF_BLOCK> out(stage, nbr, p, s);
     auto fluid_entry = [](int t) { return t; };
     auto solid_entry = [](int u) { return -1 - u; };
-    int next = 0, row = 0, a_next = 0, b_next = 0, s_next = 0, e_next = 0;
-    auto bounds = [&](int r) {
-        for (; r < 9; r++) {
-            const int y = yy + r / 3 - 1, x = xx + r % 3 - 1;
-            if (y < 0 || y >= p.gy || x < 0 || x >= p.gx) continue;
-            row = y * slab + x * p.gz;
-            a_next = fstart[row + z0];
-            b_next = fstart[row + z1 + 1];
-            if (near) {
-                s_next = sstart[row + z0];
-                e_next = sstart[row + z1 + 1];
+    // this lane's rows: two or three of the nine
+    const int q0 = G == 1 ? 0 : (g ? 2 * g + 1 : 0), q1 = G == 1 ? 9 : 2 * g + 3;
+    auto walk = [&](auto& out) {
+        int next = 0, row = 0, a_next = 0, b_next = 0, s_next = 0, e_next = 0;
+        auto bounds = [&](int r) {
+            for (; r < q1; r++) {
+                const int y = yy + r / 3 - 1, x = xx + r % 3 - 1;
+                if (y < 0 || y >= p.gy || x < 0 || x >= p.gx) continue;
+                row = y * slab + x * p.gz;
+                a_next = fstart[row + z0];
+                b_next = fstart[row + z1 + 1];
+                if (near) {
+                    s_next = sstart[row + z0];
+                    e_next = sstart[row + z1 + 1];
+                }
+                break;
             }
-            break;
+            next = r;
+        };
+        bounds(q0);
+        while (next < q1) {
+            const int a = a_next, b = b_next, sa = s_next, sb = e_next, r0 = row;
+            bounds(next + 1);
+            if (sa == sb) {
+                walk_span(xs, a, b, self, p.h2, out, fluid_entry);
+            } else if (a == b) {
+                walk_span(solid, sa, sb, self, p.h2, out, solid_entry);
+            } else {
+                int f0 = a, s0 = sa;
+                for (int c = r0 + z0; c <= r0 + z1; c++) {
+                    const int f1 = fstart[c + 1], s1 = sstart[c + 1];
+                    walk_span(xs, f0, f1, self, p.h2, out, fluid_entry);
+                    walk_span(solid, s0, s1, self, p.h2, out, solid_entry);
+                    f0 = f1;
+                    s0 = s1;
+                }
+            }
         }
-        next = r;
     };
-    bounds(0);
-    while (next < 9) {
-        const int a = a_next, b = b_next, sa = s_next, sb = e_next, r0 = row;
-        bounds(next + 1);
-        if (sa == sb) {
-            walk_span(xs, a, b, self, p.h2, out, fluid_entry);
-        } else if (a == b) {
-            walk_span(solid, sa, sb, self, p.h2, out, solid_entry);
-        } else {
-            int f0 = a, s0 = sa;
-            for (int c = r0 + z0; c <= r0 + z1; c++) {
-                const int f1 = fstart[c + 1], s1 = sstart[c + 1];
-                walk_span(xs, f0, f1, self, p.h2, out, fluid_entry);
-                walk_span(solid, s0, s1, self, p.h2, out, solid_entry);
-                f0 = f1;
-                s0 = s1;
-            }
-        }
+    StagedList<STAGE, REF_BLOCK, G> out(stage, nbr, p, s);
+    walk(out);
+    int off, c_n = group_offset<G>(out.count(), off);
+    out.write(off);
+    if (G > 1 && out.extra) {
+        LateEntries<STAGE> late{nbr + s, (size_t)p.n, off, p.max_nbrs, 0};
+        walk(late);
     }
-    int c_n = out.close();
     if (c_n > p.max_nbrs) {
         set_status(status, ST_NBR_OVERFLOW);
         c_n = p.max_nbrs;
     }
-    cnt[s] = c_n;
+    if (g == 0) cnt[s] = c_n;
 }
 
 __device__ __forceinline__ float4 nbr_pos(int j, const float4* __restrict__ xs,
@@ -308,6 +321,13 @@ __global__ void k_delta_ref(StepParams p, const float4* __restrict__ xs, float4*
 
 static inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
+// Up to this many particles a list is built by four lanes.  Measured, us a step
+// with one lane / with four: 3,000 particles of kernel radius 1.55 46.7 / 43.1,
+// 10,000 47.2 / 45.2 (of radius 2.0 66.1 / 60.9), 20,000 47.1 / 46.1, 40,000
+// 48.7 / 55.2, 100,000 67.9 / 79.5: with more particles than lanes at work the
+// group's idle lanes and second walks cost more than the shorter chain gives.
+constexpr int REF_LISTS_GROUP_MAX = 16000;
+
 void launch_predict_ref(const StepParams& p, const float4* x, float4* v, float4* xs, int* key,
                         int* rank, int* count, int* status, cudaStream_t st) {
     if (p.n <= 0) return;
@@ -324,8 +344,12 @@ void launch_lists_ref(const StepParams& p, const float4* xs, const int* key, con
                       const float4* solid, const int* sstart, int* nbr, int* cnt, int* status,
                       cudaStream_t st) {
     if (p.n <= 0) return;
-    launch_k(k_lists_ref, blocks_for(p.n, REF_BLOCK), REF_BLOCK, st, pdl_enabled(), p, xs, key, fstart, solid, sstart, nbr,
-             cnt, status);
+    if (p.n <= REF_LISTS_GROUP_MAX)
+        launch_k(k_lists_ref<4>, blocks_for(p.n, REF_BLOCK / 4), REF_BLOCK, st, pdl_enabled(), p, xs, key, fstart, solid,
+                 sstart, nbr, cnt, status);
+    else
+        launch_k(k_lists_ref<1>, blocks_for(p.n, REF_BLOCK), REF_BLOCK, st, pdl_enabled(), p, xs, key, fstart, solid,
+                 sstart, nbr, cnt, status);
 }
 
 void launch_lambda_ref(const StepParams& p, const float4* xs, const int* id, const int* nbr,

@@ -35,7 +35,12 @@ __device__ __forceinline__ int cell_ref(const StepParams& p, float x, float y, f
 // the pointer (a refused one is overwritten by the next) where a store to
 // the row under a branch would run the branch for the whole warp whenever
 // one lane accepts.  Entries past CAP (rare) go to their rows at once.
-template <int CAP, int B>
+//
+// G lanes may build one particle's list together, each a stretch of the walk:
+// a lane's place in the list is known when all have finished, so entries past
+// CAP are only counted, and a lane that has some walks its stretch again
+// (LateEntries).
+template <int CAP, int B, int G>
 struct StagedList {
     int* first;  // this thread's entry 0
     int* at;     // its next entry
@@ -54,17 +59,48 @@ struct StagedList {
             *at = e;
             at += B;
         } else {
-            if (CAP + extra < max_nbrs) row[(size_t)(CAP + extra) * n] = e;
+            if (G == 1 && CAP + extra < max_nbrs) row[(size_t)(CAP + extra) * n] = e;
             extra++;
         }
     }
-    // the staged entries to their rows; the number accepted
-    __device__ __forceinline__ int close() {
-        const int m = (int)(at - first) / B;
-        for (int k = 0; k < min(m, max_nbrs); k++) row[(size_t)k * n] = first[k * B];
-        return m + extra;
+    __device__ __forceinline__ int count() const { return (int)(at - first) / B + extra; }
+    // the staged entries to their rows, the list's place of the first being off
+    __device__ __forceinline__ void write(int off) {
+        const int m = min((int)(at - first) / B, max_nbrs - off);
+        for (int k = 0; k < m; k++) row[(size_t)(off + k) * n] = first[k * B];
     }
 };
+
+// The entries of a lane's stretch from the CAP-th on, straight to their rows.
+template <int CAP>
+struct LateEntries {
+    int* row;
+    size_t n;
+    int at, max_nbrs, seen;  // at: the place of the stretch's first entry
+    __device__ __forceinline__ bool room(int) const { return false; }
+    __device__ __forceinline__ void put(int, bool) {}
+    __device__ __forceinline__ void push(int e) {
+        if (seen >= CAP && at + seen < max_nbrs) row[(size_t)(at + seen) * n] = e;
+        seen++;
+    }
+};
+
+// Sum of the counts c of a group of G lanes; off: of the lanes before this one.
+template <int G>
+__device__ __forceinline__ int group_offset(int c, int& off) {
+    off = 0;
+    if (G == 1) return c;
+    const int g = threadIdx.x % G, lane0 = (threadIdx.x & 31) - g;
+    const unsigned mask = ((1u << G) - 1u) << lane0;
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < G; j++) {
+        const int cj = __shfl_sync(mask, c, lane0 + j);
+        off += j < g ? cj : 0;
+        total += cj;
+    }
+    return total;
+}
 
 // The particles of slots [t0, t1) of pos within h of self, in slot order,
 // entry(t) listed for each: SPAN_W positions are loaded together (past t1 too:

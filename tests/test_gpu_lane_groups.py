@@ -1,0 +1,63 @@
+"""Scenes on both sides of the sizes up to which the reference-semantics list
+builds and the sand substeps give a particle four lanes: dense clouds whose
+lists leave the staged entries of either form, cut at a capacity, beside static
+particles.  Bit for bit against the oracle."""
+import numpy as np
+import pytest
+
+from conftest import phys_params
+
+pytestmark = pytest.mark.gpu
+
+
+def _cloud(n, spacing, seed):
+    rng = np.random.default_rng(seed)
+    a = int(np.ceil(n ** (1 / 3)))
+    i = np.arange(n)
+    x = np.stack([i // a % a, i // (a * a), i % a], 1) * spacing + 1.5
+    x = (x + rng.uniform(-0.3, 0.3, x.shape) * spacing).astype(np.float32)
+    side = int(np.ceil(a * spacing)) + 4
+    s = (rng.uniform(0.05, 0.95, (n // 50, 3)) * side).astype(np.float32)
+    return x, rng.normal(0, 0.5, x.shape).astype(np.float32), s, (side, side, side)
+
+
+@pytest.mark.parametrize("n,spacing,cap", [(16_000, 0.7, 128), (16_001, 0.7, 128), (45_000, 0.65, 128),
+                                           (45_001, 0.65, 128), (45_000, 0.8, 17), (45_001, 0.8, 17)])
+def test_sand_step(orc, n, spacing, cap):
+    from lustrine_gb300 import PbfSim, sand_params
+    x, v, s, domain = _cloud(n, spacing, n)
+    ctl = orc.sand_controls(prev_attract=False, diameter=1.0)
+    p = phys_params(orc.reference_params(*domain, 0.5, 3.1))
+    o = orc.sand_step(p, ctl, np.float32(1 / 60), x, v, np.zeros(n, np.int32), solid=s, cap=256)
+    with PbfSim(sand_params(*domain, kernel_radius_scale=3.1, max_neighbors=cap), n, len(s)) as sim:
+        sim.upload(x, v, s)
+        sim.step(1 / 60)
+        cnt, idx = sim.neighbors(cap=cap)
+        full = [r[:c][r[:c] != k] for k, (c, r) in enumerate(zip(o["nbr_count"], o["nbr_idx"]))]
+        assert all(np.array_equal(idx[k, :cnt[k]], full[k][:cap]) for k in range(n))
+        if cap >= max(len(r) for r in full):
+            gx, gv, _, _ = sim.download()
+            assert np.array_equal(gx, o["x"]) and np.array_equal(gv, o["v"]) and sim.status() == 0
+        else:
+            assert cap == 17 and sim.status() == 4
+
+
+@pytest.mark.parametrize("n,spacing,cap", [(16_000, 0.8, 200), (16_001, 0.8, 200), (16_000, 0.8, 17), (16_001, 0.8, 17)])
+def test_reference_lists(orc, n, spacing, cap):
+    from lustrine_gb300 import PbfSim, reference_params
+    x, v, s, domain = _cloud(n, spacing, n)
+    ref = phys_params(orc.reference_params(*domain, 0.5, 3.1))
+    ref.jacobi = 1
+    o = orc.compat_step(ref, 0.01, x, v, solid=s, cap=256)
+    p = phys_params(reference_params(*domain, 0.5, 3.1))
+    p.max_neighbors = cap
+    with PbfSim(p, n, len(s)) as sim:
+        sim.upload(x, v, s)
+        sim.step(0.01)
+        cnt, idx = sim.neighbors(cap=cap)
+        assert np.array_equal(cnt, np.minimum(o["nbr_count"], cap))
+        assert all(np.array_equal(idx[k, :cnt[k]], o["nbr_idx"][k, :cnt[k]]) for k in range(n))
+        if cap == 200:
+            assert np.array_equal(sim.lambdas(), o["lambdas"][:n]) and sim.status() == 0
+        else:
+            assert sim.status() == 4
