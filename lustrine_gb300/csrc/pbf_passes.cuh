@@ -147,8 +147,8 @@ __device__ __forceinline__ unsigned record_entry(const uint4& r, int k) {
 // whenever a lane accepts.  That pays for rows of several particles a cell
 // (262,144 particles on voxels, 1.6 a cell: 35.5 us with the first lambda
 // summed in the branch, 31.9 like this, 32.2 with the store in it), not for
-// compact lists at unit density (2 M particles: 105 against 101 us) or one-cell
-// buckets (1 M particles hashed: 183 against 177 us).
+// compact lists at unit density (2 M particles: 105 against 101 us) or hashed
+// rows (1 M particles: 120 against 113 us).
 constexpr int COMPACT_STRIDE = 9;
 template <int FORMAT, int B, bool STAGED>
 struct StagedEntries {
@@ -312,37 +312,65 @@ __device__ __forceinline__ void walk_range(const StepParams& p, const float4& se
     }
 }
 
-// One cell of the stencil on a hashed grid: the particles of its bucket's slots
-// [t0, t1), kept only if they belong to that cell (packed).  code: the entry's
-// cell code and solid flag.  (The paired subtraction and shift keep the build at
-// 48 registers, 1 M particles in 178 us; one axis at a time it took 56 and 201.)
-template <bool MIXED, class L>
-__device__ __forceinline__ void walk_bucket(const StepParams& p, const float4& self, int skip, const float4* pos,
-                                            const int* __restrict__ cells, int packed, int t0, int t1, int code,
-                                            L& out) {
+// One stencil row on a hashed grid, the cells z0..z1 of (x, y): one slot range
+// (two where the table's end cuts it), tested in slot order, W candidates
+// loaded together.  A candidate belongs to the row if its packed cell is k
+// cells above z0's: lines that share buckets put other cells' particles in the
+// range.  code: the entry's cell code of the row (dx, dy; dz = 0) and its solid
+// flag; zc: the particle's own z.  Bound by instruction issue (1 M particles,
+// 16 blobs, first lambda included: a walk of each cell's bucket took 173 us
+// mixed and 152 compact; this one 113 and 86; one candidate at a time 128 and
+// 99).
+template <bool MIXED, bool CODES, class L>
+__device__ __forceinline__ void walk_hashed_row(const StepParams& p, const CellPack& cp, const float4& self, int skip,
+                                                int x, int y, int z0, int z1, int zc, const float4* pos,
+                                                const int* __restrict__ cells, const int* __restrict__ start, int code,
+                                                L& out) {
+    constexpr int W = 2;
     const f32x2 sxy = pack2(self.x, self.y);
     const f32x2 shift = pack2(axis_shift(p.cell, code, 25), axis_shift(p.cell, code, 27));
-    const float shift_z = axis_shift(p.cell, code, 29);
-    for (int t = t0; t < t1; t++) {
-        const ulonglong2 o = reinterpret_cast<const ulonglong2*>(pos)[t];
-        f32x2 dxy = sub2(sxy, o.x);
-        float dz = __fsub_rn(self.z, lo2(o.y));
-        if (MIXED) {
-            dxy = add2(dxy, shift);
-            dz = __fadd_rn(dz, shift_z);
+    while (z0 <= z1) {
+        const int bucket = cell_bucket(make_int3(x, y, z0), p.hash_bits);
+        const int m = min(z1 + 1 - z0, (1 << p.hash_bits) - bucket), dz0 = z0 - zc;
+        const int t0 = start[bucket], t1 = start[bucket + m];
+        const unsigned packed = pack_bits(cp, make_int3(x, y, z0));
+        const int row_code = code + (CODES ? (dz0 + 1) << 29 : 0);
+        for (int t = t0; t < t1; t += W) {
+            int tw[W], e[W];
+            unsigned k[W];
+            ulonglong2 o[W];
+            bool in[W];
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                tw[w] = w ? min(t + w, t1 - 1) : t;
+                k[w] = (unsigned)__ldg(&cells[tw[w]]) - packed;
+                o[w] = reinterpret_cast<const ulonglong2*>(pos)[tw[w]];
+            }
+#pragma unroll
+            for (int w = 0; w < W; w++) {
+                k[w] = __funnelshift_r(k[w], k[w], cp.bz_shift);  // another x or y: above any k
+                f32x2 dxy = sub2(sxy, o[w].x);
+                float dz = __fsub_rn(self.z, lo2(o[w].y));
+                if (MIXED) {
+                    dxy = add2(dxy, shift);
+                    dz = __fmaf_rn(-(float)(dz0 + (int)k[w]), p.cell, dz);  // by -1, 0 or 1: one rounding
+                }
+                e[w] = tw[w] + row_code + (CODES ? (int)(k[w] << 29) : 0);
+                in[w] = (w == 0 || t + w < t1) && tw[w] != skip && k[w] < (unsigned)m &&
+                        dot3e(lo2(dxy), hi2(dxy), dz) <= p.h2;
+            }
+            out.take(p, e, in);
         }
-        const int e[1] = {t + code};
-        const bool in[1] = {t != skip && __ldg(&cells[t]) == packed && dot3e(lo2(dxy), hi2(dxy), dz) <= p.h2};
-        out.take(p, e, in);
+        z0 += m;
     }
 }
 
 // The stencil's candidates of fluid slot s in cell c, in list order, offered to
 // out: on a dense grid the nine rows (with the static particles of each row
 // after its fluid ones where the neighbourhood holds some, near); on a hashed
-// grid the cells' buckets.  CODES: entries with cell codes (column lists).  A
-// row's bounds are loaded just before its walk (fewer live registers, more
-// resident warps), those of a row's three buckets together.
+// grid the rows' bucket ranges.  CODES: entries with cell codes (column lists).
+// A row's bounds are loaded just before its walk (fewer live registers, more
+// resident warps).
 template <bool MIXED, bool HASHED, bool SOLIDS, bool CODES, class L>
 __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack& cp, const float4& self, int s,
                                              const int3& c, const Geo& g, const float4* xs,
@@ -378,36 +406,19 @@ __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack
         // cells past the packed field widths hold no particle; the dense
         // walk's entry order: a row's fluid cells, then its solid cells
         const int z0 = max(c.z - 1, 0), z1 = min(min(c.z + 1, g.gz - 1), (int)cp.mz);
+#pragma unroll 1
         for (int dy = -1; dy <= 1; dy++) {
             const int y = c.y + dy;
             if (y < 0 || y >= g.gy || y > (int)cp.my) continue;
+#pragma unroll 1
             for (int dx = -1; dx <= 1; dx++) {
                 const int x = c.x + dx;
                 if (x < 0 || x >= g.gx || x > (int)cp.mx) continue;
-                int a[3], b[3];
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    a[k] = b[k] = 0;
-                    if (z0 + k <= z1) {
-                        const int bucket = cell_bucket(make_int3(x, y, z0 + k), p.hash_bits);
-                        a[k] = fstart[bucket];
-                        b[k] = fstart[bucket + 1];
-                    }
-                }
-                const int packed = (int)pack_bits(cp, make_int3(x, y, z0));
-                const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) | ((z0 - c.z + 1) << 29) : 0;
-                const int next_code = CODES ? 1 << 29 : 0;
-#pragma unroll
-                for (int k = 0; k < 3; k++)
-                    walk_bucket<MIXED>(p, self, s, xs, cell_sorted, packed + (k << cp.bz_shift), a[k], b[k],
-                                       code + k * next_code, out);
+                const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) : 0;
+                walk_hashed_row<MIXED, CODES>(p, cp, self, s, x, y, z0, z1, c.z, xs, cell_sorted, fstart, code, out);
                 if (SOLIDS && near)
-                    for (int z = z0; z <= z1; z++) {
-                        const int bucket = cell_bucket(make_int3(x, y, z), p.hash_bits);
-                        walk_bucket<MIXED>(p, self, -1, solid, solid_cell, packed + ((z - z0) << cp.bz_shift),
-                                           sstart[bucket], sstart[bucket + 1],
-                                           (code + ((z - z0) << 29)) | (int)0x80000000u, out);
-                    }
+                    walk_hashed_row<MIXED, CODES>(p, cp, self, -1, x, y, z0, z1, c.z, solid, solid_cell, sstart,
+                                                  code | (int)0x80000000u, out);
             }
         }
     }
@@ -436,7 +447,7 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
     using Staged = StagedEntries<FORMAT, B, FORMAT == L_COLUMN && !HASHED>;
     __shared__ unsigned stage[Staged::WORDS];
     // the cell shifts of the entries: from a table on a dense grid, formed per
-    // entry on a hashed one (whose walk leaves it no registers: 200 against 177 us)
+    // entry on a hashed one (whose walk leaves it no registers)
     constexpr bool TABLE = MIXED && !HASHED;
     __shared__ float4 shift_tab[TABLE ? 64 : 1];
     pdl_wait();
