@@ -217,6 +217,23 @@ inline void launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t
 void set_pdl(bool on);
 bool pdl_enabled();
 
+// Sum of the counts c of a group of G lanes; off: of the lanes before this one.
+template <int G>
+__device__ __forceinline__ int group_offset(int c, int& off) {
+    off = 0;
+    if (G == 1) return c;
+    const int g = threadIdx.x % G, lane0 = (threadIdx.x & 31) - g;
+    const unsigned mask = ((1u << G) - 1u) << lane0;
+    int total = 0;
+#pragma unroll
+    for (int j = 0; j < G; j++) {
+        const int cj = __shfl_sync(mask, c, lane0 + j);
+        off += j < g ? cj : 0;
+        total += cj;
+    }
+    return total;
+}
+
 // PBF neighbour lists: rows allocated = max_nbrs rounded up to LIST_PAD_MAX;
 // the sentinel slot n sits at SENTINEL_POS on every axis.
 constexpr int LIST_PAD_MAX = 8;

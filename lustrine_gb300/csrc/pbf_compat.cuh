@@ -85,23 +85,6 @@ struct LateEntries {
     }
 };
 
-// Sum of the counts c of a group of G lanes; off: of the lanes before this one.
-template <int G>
-__device__ __forceinline__ int group_offset(int c, int& off) {
-    off = 0;
-    if (G == 1) return c;
-    const int g = threadIdx.x % G, lane0 = (threadIdx.x & 31) - g;
-    const unsigned mask = ((1u << G) - 1u) << lane0;
-    int total = 0;
-#pragma unroll
-    for (int j = 0; j < G; j++) {
-        const int cj = __shfl_sync(mask, c, lane0 + j);
-        off += j < g ? cj : 0;
-        total += cj;
-    }
-    return total;
-}
-
 // The particles of slots [t0, t1) of pos within h of self, in slot order,
 // entry(t) listed for each: SPAN_W positions are loaded together (past t1 too:
 // the buffers are SPAN_PAD longer), then tested in order.  The squared

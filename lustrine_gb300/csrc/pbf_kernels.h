@@ -122,6 +122,19 @@ void launch_xsph(bool mixed, const Tuning& tu, const StepParams& p, const CellPa
                  const float4* xs, const float4* v_in, const int* nbr, const int* cnt,
                  const int* key_sorted, float4* x_out, float4* v_out, float4* xs_next, int* key,
                  int* rank, int* count, int* cellk, int* tile_count, cudaStream_t st);
+// Up to this many particles a dense grid's list build gives each four lanes (16-bit
+// records and column lists): a small scene has fewer warps than the GPU has
+// schedulers, and one lane's nine rows are a chain of dependent loads.  The line
+// lies where the groups' blocks still run in one wave.  Measured, us a step with
+// one lane / with four:
+//     n        compact        on voxels      mixed
+//     3,000    33.4 / 28.9    46.9 / 42.6    48.1 / 44.4
+//     10,000   33.8 / 30.3    47.9 / 44.4    50.8 / 45.7
+//     20,000   35.8 / 32.4    53.6 / 48.7    53.4 / 49.1
+//     40,000   36.1 / 35.5    55.3 / 51.9    52.9 / 57.2
+//     60,000   40.2 / 42.1    57.9 / 60.5    57.3 / 66.3
+constexpr int LISTS_GROUP_MAX = 45000;
+constexpr int LISTS_GROUP_MAX_MIXED = 30000;
 // The same passes over compact lists (p.rec set; pbf_compact.cu).  B: the
 // list build's block size; p.pad: the passes' largest chunk.
 void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4* xs, const int* key_sorted,

@@ -162,12 +162,13 @@ struct StagedEntries {
     int* row;  // nbr + s
     int base;  // 16-bit entries: the scene's first slot
     int extra = 0;  // entries past CAP
-    __device__ __forceinline__ StagedEntries(unsigned* smem, int* nbr, const StepParams& p, int s, int slot0)
+    __device__ __forceinline__ StagedEntries(unsigned* smem, int at_thread, int* nbr, const StepParams& p, int s,
+                                             int slot0)
         : row(nbr + s), base(slot0) {
         if (FORMAT == L_C16)
-            first = reinterpret_cast<T*>(smem + COMPACT_STRIDE * threadIdx.x);
+            first = reinterpret_cast<T*>(smem + COMPACT_STRIDE * at_thread);
         else
-            first = reinterpret_cast<T*>(smem) + threadIdx.x;
+            first = reinterpret_cast<T*>(smem) + at_thread;
         at = first;
         // places past the count hold the sentinel in the records
         if (FORMAT == L_C16) {
@@ -201,6 +202,15 @@ struct StagedEntries {
             for (int u = 0; u < W; u++)
                 if (in[u]) push(p, e[u]);
         }
+    }
+    // entry k set by itself, and the number of entries then (lists built by a group)
+    __device__ __forceinline__ void place(const StepParams& p, int k, int e) {
+        if (k < CAP) first[k * STEP] = (T)(FORMAT == L_C16 ? e - base : e);
+        else if (k < p.max_nbrs) row[(size_t)(k - ROW0) * p.n] = e;
+    }
+    __device__ __forceinline__ void set_count(int c) {
+        at = first + min(c, CAP) * STEP;
+        extra = max(c - CAP, 0);
     }
     __device__ __forceinline__ int staged() const { return (int)(at - first) / STEP; }
     __device__ __forceinline__ int count() const { return staged() + extra; }
@@ -244,6 +254,39 @@ struct StagedEntries {
         p.rec[s] = r;
         if (c_n > ROW0 - RecordFormat<FORMAT>::EXT) p.rec2[s] = r2;
         for (int k = c_n - ROW0; k > 0 && k % p.pad != 0; k++) row[(size_t)k * p.n] = p.n;
+    }
+};
+
+// One lane's part of a list that a group of lanes builds: the accepted
+// candidates of its rows in order, k at [k][thread]; those past CAP are only
+// counted, and LatePart collects them once the lane's place is known.
+template <int B>
+struct LanePart {
+    static constexpr int CAP = 12;
+    int* first;
+    int c = 0;
+    template <int W>
+    __device__ __forceinline__ void take(const StepParams&, const int (&e)[W], const bool (&in)[W]) {
+#pragma unroll
+        for (int u = 0; u < W; u++)
+            if (in[u]) {
+                if (c < CAP) first[c * B] = e[u];
+                c++;
+            }
+    }
+};
+template <int CAP, class Staged>
+struct LatePart {
+    Staged& list;
+    int off, c;
+    template <int W>
+    __device__ __forceinline__ void take(const StepParams& p, const int (&e)[W], const bool (&in)[W]) {
+#pragma unroll
+        for (int u = 0; u < W; u++)
+            if (in[u]) {
+                if (c >= CAP) list.place(p, off + c, e[u]);
+                c++;
+            }
     }
 };
 
@@ -371,7 +414,7 @@ __device__ __forceinline__ void walk_hashed_row(const StepParams& p, const CellP
 // grid the rows' bucket ranges.  CODES: entries with cell codes (column lists).
 // A row's bounds are loaded just before its walk (fewer live registers, more
 // resident warps).
-template <bool MIXED, bool HASHED, bool SOLIDS, bool CODES, class L>
+template <bool MIXED, bool HASHED, bool SOLIDS, bool CODES, int G = 1, class L>
 __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack& cp, const float4& self, int s,
                                              const int3& c, const Geo& g, const float4* xs,
                                              const int* __restrict__ cell_sorted, const int* __restrict__ fstart,
@@ -380,26 +423,36 @@ __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack
     if constexpr (!HASHED) {
         // 4 candidates at a time for column lists, 2 for compact ones (their
         // build is held to 40 registers)
-        constexpr int W = CODES ? 4 : 2;
+        constexpr int W = CODES || G > 1 ? 4 : 2;
         const int slab = g.gx * g.gz;
         const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, g.gz - 1);
+        auto row_of = [&](int dy, int y, int dx) {
+            const int x = c.x + dx;
+            if (x < 0 || x >= g.gx) return;
+            const int row = g.off + y * slab + x * g.gz;
+            const int i1 = row + z0 + 1, i2 = row + min(z0 + 2, z1 + 1);  // the second and third cell
+            const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) | (1 << 29) : 0;
+            walk_range<MIXED, W>(p, self, s, xs, fstart[row + z0], fstart[row + z1 + 1], MIXED ? fstart[i1] : 0,
+                                 MIXED ? fstart[i2] : 0, z0 - c.z, code, out);
+            if (SOLIDS && near)
+                walk_range<MIXED, W>(p, self, -1, solid, sstart[row + z0], sstart[row + z1 + 1],
+                                     MIXED ? sstart[i1] : 0, MIXED ? sstart[i2] : 0, z0 - c.z,
+                                     code | (int)0x80000000u, out);
+        };
+        if constexpr (G == 4) {  // a lane's two or three rows
+            const int lane = threadIdx.x % G;
 #pragma unroll 1
-        for (int dy = -1; dy <= 1; dy++) {
-            const int y = c.y + dy;
-            if (y < 0 || y >= g.gy) continue;
+            for (int r = lane ? 2 * lane + 1 : 0; r < 2 * lane + 3; r++) {
+                const int dy = r / 3 - 1, y = c.y + dy;
+                if (y >= 0 && y < g.gy) row_of(dy, y, r % 3 - 1);
+            }
+        } else {
 #pragma unroll 1
-            for (int dx = -1; dx <= 1; dx++) {
-                const int x = c.x + dx;
-                if (x < 0 || x >= g.gx) continue;
-                const int row = g.off + y * slab + x * g.gz;
-                const int i1 = row + z0 + 1, i2 = row + min(z0 + 2, z1 + 1);  // the second and third cell
-                const int code = CODES ? ((dx + 1) << 25) | ((dy + 1) << 27) | (1 << 29) : 0;
-                walk_range<MIXED, W>(p, self, s, xs, fstart[row + z0], fstart[row + z1 + 1], MIXED ? fstart[i1] : 0,
-                                     MIXED ? fstart[i2] : 0, z0 - c.z, code, out);
-                if (SOLIDS && near)
-                    walk_range<MIXED, W>(p, self, -1, solid, sstart[row + z0], sstart[row + z1 + 1],
-                                         MIXED ? sstart[i1] : 0, MIXED ? sstart[i2] : 0, z0 - c.z,
-                                         code | (int)0x80000000u, out);
+            for (int dy = -1; dy <= 1; dy++) {
+                const int y = c.y + dy;
+                if (y < 0 || y >= g.gy) continue;
+#pragma unroll 1
+                for (int dx = -1; dx <= 1; dx++) row_of(dy, y, dx);
             }
         }
     } else {
@@ -435,7 +488,9 @@ __device__ __forceinline__ void walk_stencil(const StepParams& p, const CellPack
 // together (in the cache from the walk); a list cut at the capacity walks once
 // more to sum the dropped entries after the listed ones, so that the terms
 // and their order do not depend on the capacity or the format.
-template <bool MIXED, bool HASHED, bool FRAME, int FORMAT, bool SOLIDS, int B>
+// G = 4 (dense grids): four lanes share a particle's rows, each collecting its
+// part; then the first of them holds the list and goes on alone.
+template <bool MIXED, bool HASHED, bool FRAME, int FORMAT, bool SOLIDS, int B, int G = 1>
 __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack& cp, float4* __restrict__ xs,
                                              const int* __restrict__ key_sorted, const int* __restrict__ cell_sorted,
                                              const int* __restrict__ fstart, const float4* __restrict__ solid,
@@ -444,7 +499,7 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
                                              int* status) {
     static_assert(FORMAT == L_COLUMN || (!MIXED && !SOLIDS), "compact lists");
     constexpr bool CODES = FORMAT == L_COLUMN;
-    using Staged = StagedEntries<FORMAT, B, FORMAT == L_COLUMN && !HASHED>;
+    using Staged = StagedEntries<FORMAT, B / G, FORMAT == L_COLUMN && !HASHED>;
     __shared__ unsigned stage[Staged::WORDS];
     // the cell shifts of the entries: from a table on a dense grid, formed per
     // entry on a hashed one (whose walk leaves it no registers)
@@ -452,7 +507,7 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
     __shared__ float4 shift_tab[TABLE ? 64 : 1];
     pdl_wait();
     if (TABLE) fill_shift_table(p, shift_tab);
-    const int s = blockIdx.x * B + threadIdx.x;
+    const int s = (blockIdx.x * B + threadIdx.x) / G;
     if (s >= p.n) return;
     const float4 self = xs[s];
     const Geo g = geo_slot(p, s);
@@ -460,11 +515,32 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
     constexpr bool KAHAN = MIXED || FRAME;
     const int3 c = (MIXED || HASHED || FRAME) ? slot_cell(p, cp, g, key_sorted, cell_sorted, s)
                                               : plain_cell(p, g, self.x, self.y, self.z);
-    Staged out(stage, nbr, p, s, g.slot0);
+    Staged out(stage, threadIdx.x / G, nbr, p, s, g.slot0);
     // static particles only where the cell's neighbourhood holds some
     const bool near = SOLIDS && p.ns > 0 && p.solid_near && __ldg(&p.solid_near[__ldg(&key_sorted[s])]);
-    walk_stencil<MIXED, HASHED, SOLIDS, CODES>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid, solid_cell,
-                                               sstart, near, out);
+    if constexpr (G == 1) {
+        walk_stencil<MIXED, HASHED, SOLIDS, CODES>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid, solid_cell,
+                                                   sstart, near, out);
+    } else {
+        using Lane = LanePart<B>;
+        __shared__ int part[Lane::CAP * B];
+        Lane mine{part + threadIdx.x};
+        walk_stencil<MIXED, HASHED, SOLIDS, CODES, G>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid,
+                                                      solid_cell, sstart, near, mine);
+        int off;
+        const int total = group_offset<G>(mine.c, off);
+        const unsigned group = ((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1));
+        __syncwarp(group);  // the list's sentinel entries are set
+        for (int k = 0; k < min(mine.c, Lane::CAP); k++) out.place(p, off + k, mine.first[k * B]);
+        if (mine.c > Lane::CAP) {
+            LatePart<Lane::CAP, Staged> late{out, off, 0};
+            walk_stencil<MIXED, HASHED, SOLIDS, CODES, G>(p, cp, self, s, c, g, xs, cell_sorted, fstart, solid,
+                                                          solid_cell, sstart, near, late);
+        }
+        __syncwarp(group);
+        if (threadIdx.x % G) return;
+        out.set_count(total);
+    }
     int c_n = out.count();
     const int m = min(c_n, p.max_nbrs);
     LambdaAcc a = lambda_init(p);
@@ -497,7 +573,7 @@ __device__ __forceinline__ void lists_lambda(const StepParams& p, const CellPack
     if (rho) rho[s] = density_of(p, a);
 }
 
-template <bool MIXED, bool HASHED, int B, bool FRAME = false>
+template <bool MIXED, bool HASHED, int B, bool FRAME = false, int G = 1>
 __global__ void __launch_bounds__(B) k_lists_lambda(StepParams p, CellPack cp, float4* __restrict__ xs,
                                                     const int* __restrict__ key_sorted,
                                                     const int* __restrict__ cell_sorted,
@@ -507,8 +583,19 @@ __global__ void __launch_bounds__(B) k_lists_lambda(StepParams p, CellPack cp, f
                                                     const int* __restrict__ sstart,
                                                     int* __restrict__ nbr, int* __restrict__ cnt,
                                                     float* __restrict__ rho, int* status) {
-    lists_lambda<MIXED, HASHED, FRAME, 0, true, B>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
+    lists_lambda<MIXED, HASHED, FRAME, 0, true, B, G>(p, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
                                                    sstart, nbr, cnt, rho, status);
+}
+
+// Compact 16-bit lists by four lanes a particle (small dense scenes).
+template <int B, bool FRAME>
+__global__ void __launch_bounds__(B) k_lists_compact_group(StepParams p, CellPack cp, float4* __restrict__ xs,
+                                                           const int* __restrict__ key_sorted,
+                                                           const int* __restrict__ cell_sorted,
+                                                           const int* __restrict__ fstart, int* __restrict__ nbr,
+                                                           int* __restrict__ cnt, float* __restrict__ rho, int* status) {
+    lists_lambda<false, false, FRAME, L_C16, false, B, 4>(p, cp, xs, key_sorted, cell_sorted, fstart, nullptr, nullptr,
+                                                          nullptr, nbr, cnt, rho, status);
 }
 
 // Compact lists (no static particles, fp32 pair offsets).

@@ -1,0 +1,64 @@
+"""List builds by four lanes a particle (dense grids up to a size) against the
+hashed grid of the same scene, which always takes one: sizes on both sides of
+the lines, and clumps whose lists leave a lane's part, the staged entries and
+the capacity.  The same candidates in the same order, so the first step agrees
+bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _scene(n, spacing, solids):
+    rng = np.random.default_rng(n)
+    a = int(np.ceil(n ** (1 / 3)))
+    i = np.arange(n)
+    x = np.stack([i // a % a, i // (a * a), i % a], 1) * spacing + 2.0
+    x = (x + rng.uniform(-0.3, 0.3, x.shape) * spacing).astype(np.float32)
+    side = int(np.ceil(a * spacing)) + 5
+    s = np.unique(rng.integers(1, side - 1, (max(n // 20, 40), 3)), axis=0).astype(np.float32) + 0.5
+    return x, s if solids else None, (side, side, side)
+
+
+@pytest.mark.parametrize("solids", [False, True])
+@pytest.mark.parametrize("n,precision,spacing,cap", [
+    (45_000, 0, 0.9, 64), (45_001, 0, 0.9, 64), (30_000, 1, 0.9, 64), (30_001, 1, 0.9, 64),
+    (1, 0, 1.0, 64), (333, 0, 0.5, 96), (333, 1, 0.5, 96), (1_111, 0, 0.3, 250), (1_111, 1, 0.3, 250),
+    (333, 0, 0.5, 9), (333, 1, 0.5, 9), (1_111, 0, 0.3, 61), (1_111, 1, 0.3, 61)])
+def test_first_step(n, precision, spacing, cap, solids):
+    from lustrine_gb300 import PbfSim, pbf_params
+    from lustrine_gb300._lib import GRID_DENSE, GRID_HASHED
+    x, s, domain = _scene(n, spacing, solids)
+    got = []
+    for grid in (GRID_DENSE, GRID_HASHED):
+        p = pbf_params(*domain, iterations=2, precision=precision, grid_mode=grid, max_neighbors=cap)
+        with PbfSim(p, n, 0 if s is None else len(s)) as sim:
+            sim.upload(x, None, s)
+            sim.step(1 / 60)
+            got.append(sim.download(lambdas=True, density=True) + sim.neighbors(cap=cap + 1) + (sim.status(),))  # + itself
+    dense, hashed = got
+    cut = cap in (9, 61)
+    assert dense[6] == hashed[6] == (4 if cut else 0)
+    assert dense[4].max() == cap + 1 if cut else (dense[4].max() > (48 if spacing == 0.3 else 0) or n == 1)
+    for a, b in zip(dense[:6], hashed[:6]):
+        np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("n", [45_000, 45_001, 777])
+def test_scene_frame_lists(n):
+    """The scene frame: the lists of one step are those of fp32 positions where no
+    pair lies within rounding of the radius."""
+    from lustrine_gb300 import PbfSim, pbf_params
+    x, _, domain = _scene(n, 0.9, False)
+    got = []
+    for precision in (0, 2):
+        with PbfSim(pbf_params(*domain, iterations=2, precision=precision), n) as sim:
+            sim.upload(x, None, None)
+            sim.step(1 / 60)
+            assert sim.status() == 0
+            got.append(sim.neighbors())
+    (c0, i0), (c2, i2) = got
+    assert np.mean(c0 != c2) < 1e-3
+    # the order within a row follows the slots, the same for both
+    same = c0 == c2
+    assert np.mean(np.any(i0[same] != i2[same], axis=1)) < 1e-3
