@@ -457,7 +457,8 @@ LUSTRINE_API int lustrine_pbf_profile_step(lustrine_pbf* s, float dt, double* st
 enum {
     LUSTRINE_LISTS_COLUMN = 0,       /* count + column-major 32-bit entries */
     LUSTRINE_LISTS_COMPACT = 1,      /* 16-byte records: count, scene's first slot, 6 (+8) 16-bit offsets */
-    LUSTRINE_LISTS_COMPACT_WIDE = 2  /* reported only: 16-byte records, count and 3 (+4) 32-bit slots */
+    LUSTRINE_LISTS_COMPACT_WIDE = 2  /* reported only: 16-byte records, count and 5 (+5) 24-bit slots
+                                        (3 (+4) of 32 bits from 2^24 slots on) */
 };
 typedef struct lustrine_pbf_tuning {
     int block;

@@ -1,6 +1,6 @@
-// pbf_compat.cuh -- the reference's cell mapping, shared by the
-// reference-semantics steps (fluid, pbf_compat.cu; sand, sand.cu).  Both are
-// compiled with --fmad=false.
+// pbf_compat.cuh -- the reference's cell mapping and the list entries' way
+// through shared memory, shared by the reference-semantics steps (fluid,
+// pbf_compat.cu; sand, sand.cu).  Both are compiled with --fmad=false.
 #pragma once
 
 #include "pbf_common.cuh"

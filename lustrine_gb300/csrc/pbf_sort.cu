@@ -8,9 +8,10 @@
 //   2. exclusive scan of count over all cells: tile totals, then every tile
 //      scanned from the sum of the totals before it (k_tile_sums,
 //      k_scan_tiles; grids of more than CELL_SCAN_MAX_TILES tiles scan the
-//      totals in one block in between); the standalone sort entry points use
-//      reduce / scan of the tile sums / down-sweep; the scan also zeroes
-//      count for the next step's histogram;
+//      totals in one block in between); where the offsets are not 16-byte
+//      aligned (a caller's array at the standalone sort entry points), and in
+//      set-up, reduce / scan of the tile sums / down-sweep; the scan also
+//      zeroes count for the next step's histogram;
 //   3. scatter of particle indices to start[key] + rank;
 //   4. stabilisation: atomic arrival order is arbitrary, so every cell's
 //      members are put in the order of a tie key (previous slot, or the

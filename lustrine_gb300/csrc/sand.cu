@@ -14,7 +14,7 @@
 // Step: k_sand_predict (integration, attract and blow, box clamp, cell key,
 // histogram) -> cell scan -> stable scatter/gather of x, x*, attract flags
 // into cell order -> k_sand_lists (symmetric lists in the reference's push
-// order) -> 4 x k_sand_substep; the last substep commits x, v and the flags
+// order) -> 4 x k_sand_substep (k_sand_substep_group in small scenes); the last substep commits x, v and the flags
 // back into the side the step started from.
 #include "pbf_common.cuh"
 #include "pbf_compat.cuh"
