@@ -11,9 +11,13 @@
 // range is read from a page-locked word that the histogram writes only then
 // (a copy from the device otherwise, when all words are in use).  Both are
 // shared by threads: the pool is stream-ordered, a word belongs to one call.
+// Both end with the device's context: a call after a device reset (or from a
+// second context of the device) finds that they are not its own.
 #include <atomic>
 #include <cstdio>
 #include <mutex>
+
+#include <cuda.h>
 
 #include "lustrine_gb300.h"
 #include "pbf_context.h"
@@ -27,52 +31,82 @@ constexpr unsigned long long SCRATCH_KEPT = 128ull << 20;
 constexpr int kMaxDevices = 64;
 constexpr int kWords = 64;
 
+struct DeviceScratch {
+    unsigned long long context = 0;  // the context both belong to
+    cudaMemPool_t pool = nullptr;
+    int* words = nullptr;  // page-locked, kWords ints
+    std::atomic<bool> used[kWords];
+};
 std::mutex g_lock;
-cudaMemPool_t g_pool[kMaxDevices] = {};
-int* g_words = nullptr;  // page-locked, kWords ints
-std::atomic<bool> g_word_used[kWords];
+DeviceScratch g_scratch[kMaxDevices];
 
-// The current device's scratch pool, or nullptr (the default pool serves).
-cudaMemPool_t scratch_pool() {
+// The current context's id, never used twice in a process; 0 if unknown.
+unsigned long long context_id() {
+    static const auto get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) != cudaSuccess ||
+            found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return (CUresult(CUDAAPI*)(CUcontext, unsigned long long*))f;
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// Whether the words are still page-locked memory (not after a reset).
+bool alive(const int* words) {
+    cudaPointerAttributes a = {};
+    if (cudaPointerGetAttributes(&a, words) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeHost && a.hostPointer == words;
+}
+
+bool open_scratch(DeviceScratch& d, int dev) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = SCRATCH_KEPT;
+    if (cudaMemPoolCreate(&d.pool, &props) == cudaSuccess) {
+        if (cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess &&
+            cudaHostAlloc((void**)&d.words, kWords * sizeof(int),
+                          cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess)
+            return true;
+        cudaMemPoolDestroy(d.pool);
+    }
+    cudaGetLastError();
+    return false;
+}
+
+// The current device's scratch, or nullptr (the default pool and a status word
+// on the device serve).
+DeviceScratch* device_scratch(bool create) {
     int dev = -1;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+    if (cudaFree(nullptr) != cudaSuccess) return nullptr;  // the device's context made current
+    const unsigned long long context = context_id();
+    if (!context) return nullptr;
     std::lock_guard<std::mutex> lock(g_lock);
-    if (!g_pool[dev]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        cudaMemPool_t pool = nullptr;
-        unsigned long long keep = SCRATCH_KEPT;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            cudaMemPoolDestroy(pool);
-            return nullptr;
-        }
-        g_pool[dev] = pool;
-    }
-    return g_pool[dev];
+    DeviceScratch& d = g_scratch[dev];
+    if (d.words && alive(d.words)) return d.context == context ? &d : nullptr;
+    d.words = nullptr;
+    for (auto& u : d.used) u.store(false);
+    if (!create || !open_scratch(d, dev)) return nullptr;
+    d.context = context;
+    return &d;
 }
 
 // A page-locked word of this call's own, zero; -1 when none is free.
-int take_word() {
-    {
-        std::lock_guard<std::mutex> lock(g_lock);
-        if (!g_words && cudaHostAlloc((void**)&g_words, kWords * sizeof(int),
-                                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
-            cudaGetLastError();
-            g_words = nullptr;
-            return -1;
-        }
-    }
-    for (int k = 0; k < kWords; k++) {
+int take_word(DeviceScratch* d) {
+    for (int k = 0; d && k < kWords; k++) {
         bool free = false;
-        if (g_word_used[k].compare_exchange_strong(free, true)) {
-            *(volatile int*)&g_words[k] = 0;
+        if (d->used[k].compare_exchange_strong(free, true)) {
+            *(volatile int*)&d->words[k] = 0;
             return k;
         }
     }
@@ -95,18 +129,18 @@ extern "C" int lustrine_counting_sort(int* counts, const int* keys, size_t num_p
     const int n = (int)num_positions, C = (int)num_cells;
     const size_t bytes = counting_sort_scratch_ints(n, C) * sizeof(int);
     int* scratch = nullptr;
-    cudaMemPool_t pool = scratch_pool();
-    cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)&scratch, bytes, pool, st)
+    DeviceScratch* const kept = device_scratch(true);
+    cudaError_t e = kept ? cudaMallocFromPoolAsync((void**)&scratch, bytes, kept->pool, st)
                          : cudaMallocAsync((void**)&scratch, bytes, st);
     if (e != cudaSuccess) return lgb_cuda_status(e, "cudaMallocAsync");
     CountingSortScratch w = counting_sort_scratch(scratch, n, C);
     int bad = 0;
-    const int word = take_word();
+    const int word = take_word(kept);
     // the histogram and the status word behind it start at zero
     e = cudaMemsetAsync(w.count, 0, ((size_t)C + 1) * sizeof(int), st);
     if (e == cudaSuccess) {
         int* const device_status = w.status;
-        if (word >= 0) w.status = &g_words[word];
+        if (word >= 0) w.status = &kept->words[word];
         const cudaError_t before = cudaPeekAtLastError();  // an earlier call's error is not this one's
         launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
         if (before == cudaSuccess) e = cudaPeekAtLastError();
@@ -116,8 +150,8 @@ extern "C" int lustrine_counting_sort(int* counts, const int* keys, size_t num_p
     const cudaError_t e1 = cudaFreeAsync(scratch, st);
     const cudaError_t e2 = cudaStreamSynchronize(st);
     if (word >= 0) {
-        bad = *(volatile int*)&g_words[word];
-        g_word_used[word].store(false);
+        bad = *(volatile int*)&kept->words[word];
+        kept->used[word].store(false);
     }
     if (e == cudaSuccess) e = e2 != cudaSuccess ? e2 : e1;
     if (e != cudaSuccess) return lgb_cuda_status(e, "counting_sort");
@@ -125,14 +159,8 @@ extern "C" int lustrine_counting_sort(int* counts, const int* keys, size_t num_p
 }
 
 extern "C" int lustrine_release_scratch(void) {
-    int dev = -1;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return lgb_cuda_status(e, "cudaGetDevice");
-    cudaMemPool_t pool = nullptr;
-    if (dev >= 0 && dev < kMaxDevices) {
-        std::lock_guard<std::mutex> lock(g_lock);
-        pool = g_pool[dev];
-    }
-    if (pool && (e = cudaMemPoolTrimTo(pool, 0)) != cudaSuccess) return lgb_cuda_status(e, "cudaMemPoolTrimTo");
+    DeviceScratch* const kept = device_scratch(false);
+    cudaError_t e = cudaSuccess;
+    if (kept && (e = cudaMemPoolTrimTo(kept->pool, 0)) != cudaSuccess) return lgb_cuda_status(e, "cudaMemPoolTrimTo");
     return LUSTRINE_OK;
 }
