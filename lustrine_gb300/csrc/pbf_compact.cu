@@ -12,9 +12,10 @@ void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4
                           const int* cell_sorted, const int* fstart, const float4* solid, const int* solid_cell,
                           const int* sstart, int* nbr, int* cnt, float* rho, int* status, cudaStream_t st) {
     const bool pdl = pdl_enabled();
-    if (p.n <= LISTS_GROUP_MAX && !p.hash_bits && !p.wide) {
-        launch_k(p.frame ? k_lists_compact_group<128, true> : k_lists_compact_group<128, false>, blocks_for(p.n, 32), 128,
-                 st, pdl, p, cp, xs, key_sorted, cell_sorted, fstart, nbr, cnt, rho, status);
+    if (p.n <= LISTS_GROUP_MAX_COMPACT && !p.hash_bits && !p.wide) {
+        constexpr int GB = LISTS_GROUP_BLOCK;
+        launch_k(p.frame ? k_lists_compact_group<GB, true> : k_lists_compact_group<GB, false>, blocks_for(p.n, GB / 4),
+                 GB, st, pdl, p, cp, xs, key_sorted, cell_sorted, fstart, nbr, cnt, rho, status);
         return;
     }
 #define LGB_LISTS_C(H, FR, W, BB)                                                                     \

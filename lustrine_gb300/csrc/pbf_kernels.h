@@ -123,18 +123,24 @@ void launch_xsph(bool mixed, const Tuning& tu, const StepParams& p, const CellPa
                  const int* key_sorted, float4* x_out, float4* v_out, float4* xs_next, int* key,
                  int* rank, int* count, int* cellk, int* tile_count, cudaStream_t st);
 // Up to this many particles a dense grid's list build gives each four lanes (16-bit
-// records and column lists): a small scene has fewer warps than the GPU has
-// schedulers, and one lane's nine rows are a chain of dependent loads.  The line
-// lies where the groups' blocks still run in one wave.  Measured, us a step with
-// one lane / with four:
-//     n        compact        on voxels      mixed
-//     3,000    33.4 / 28.9    46.9 / 42.6    48.1 / 44.4
-//     10,000   33.8 / 30.3    47.9 / 44.4    50.8 / 45.7
-//     20,000   35.8 / 32.4    53.6 / 48.7    53.4 / 49.1
-//     40,000   36.1 / 35.5    55.3 / 51.9    52.9 / 57.2
-//     60,000   40.2 / 42.1    57.9 / 60.5    57.3 / 66.3
-constexpr int LISTS_GROUP_MAX = 45000;
-constexpr int LISTS_GROUP_MAX_MIXED = 30000;
+// records; column lists but those of per-cell mixed positions): a small scene has
+// fewer warps than the GPU has schedulers, and one lane's nine rows are a chain of
+// dependent loads.  Measured,
+// us a step with one lane / with four:
+//     n        compact        on voxels
+//     3,000    32.3 / 28.9    46.0 / 42.1
+//     10,000   33.5 / 30.8    48.7 / 44.6
+//     20,000   35.6 / 31.7    54.6 / 48.8
+//     40,000   36.1 / 35.0    52.7 / 51.1
+// Where many contexts overlap on the GPU the lanes cost instructions and blocks:
+// 512 scenes of 1,024 to 65,536 particles, a context each, take 1.68 ms a step with
+// one lane, 1.74 with four up to 11,000 particles (256 threads a block; 1.79 with
+// 128), 2.00 up to 45,000; 96 scenes of 2,000 to 20,000 on voxels 0.45 and 0.47,
+// with per-cell mixed positions (64 registers) 0.49 and 0.56 (one by one 49.6 / 46.4
+// us at 10,000), which keep one lane.
+constexpr int LISTS_GROUP_MAX_COMPACT = 11000;
+constexpr int LISTS_GROUP_MAX_COLUMN = 20000;
+constexpr int LISTS_GROUP_BLOCK = 256;
 // The same passes over compact lists (p.rec set; pbf_compact.cu).  B: the
 // list build's block size; p.pad: the passes' largest chunk.
 void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4* xs, const int* key_sorted,

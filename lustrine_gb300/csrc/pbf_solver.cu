@@ -408,10 +408,10 @@ void launch_lists_lambda(bool mixed, const Tuning& tu, const StepParams& p, cons
     if (p.rec) {  // compact lists (pbf_compact.cu)
         launch_lists_compact(B, pp, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell, sstart, nbr, cnt,
                              rho, status, st);
-    } else if (p.n <= (mixed && !p.frame ? LISTS_GROUP_MAX_MIXED : LISTS_GROUP_MAX) && !p.hash_bits) {
-        launch_k(!mixed ? k_lists_lambda<false, false, 128, false, 4>
-                        : (p.frame ? k_lists_lambda<false, false, 128, true, 4> : k_lists_lambda<true, false, 128, false, 4>),
-                 blocks_for(p.n, 32), 128, st, pdl, pp, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
+    } else if (p.n <= LISTS_GROUP_MAX_COLUMN && !p.hash_bits && (!mixed || p.frame)) {
+        constexpr int GB = LISTS_GROUP_BLOCK;
+        launch_k(mixed ? k_lists_lambda<false, false, GB, true, 4> : k_lists_lambda<false, false, GB, false, 4>,
+                 blocks_for(p.n, GB / 4), GB, st, pdl, pp, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
                  sstart, nbr, cnt, rho, status);
     } else if (mixed && p.frame) {  // the scene frame: fp32 pair offsets, compensated sums
         if (B == 64) launch_k(k_lists_lambda<false, false, 64, true>, blocks_for(p.n, 64), 64, st, pdl, pp, cp, xs,
