@@ -14,7 +14,7 @@
 // Step: k_sand_predict (integration, attract and blow, box clamp, cell key,
 // histogram) -> cell scan -> stable scatter/gather of x, x*, attract flags
 // into cell order -> k_sand_lists (symmetric lists in the reference's push
-// order) -> 4 x k_sand_substep (k_sand_substep_group in small scenes); the last substep commits x, v and the flags
+// order) -> 4 x k_sand_substep; the last substep commits x, v and the flags
 // back into the side the step started from.
 #include "pbf_common.cuh"
 #include "pbf_compat.cuh"
@@ -351,100 +351,16 @@ __global__ void __launch_bounds__(SAND_BLOCK) k_sand_substep(
     id_commit[i] = i;
 }
 
-// The same substep with SAND_GROUP lanes a particle, for scenes whose particles
-// alone leave the schedulers without warps: the lanes test 16 entries of the list
-// together, note the contacts in list order, evaluate a contact each, and lanes
-// 0-2 subtract the x, y and z terms in order.
-constexpr int SAND_GROUP = 4;
-constexpr int GROUP_HITS = 32;   // contacts noted before they are evaluated
-constexpr int GROUP_TERMS = 16;  // terms held at once
-__global__ void __launch_bounds__(SAND_BLOCK) k_sand_substep_group(
-    StepParams p, SandParams q, const float4* __restrict__ tmp_in, float4* __restrict__ star_out,
-    const float4* __restrict__ xpre, const int* __restrict__ nbr, const int* __restrict__ cnt,
-    const float4* __restrict__ solid, float4* __restrict__ x_commit, float4* __restrict__ v_commit,
-    const int* __restrict__ att_in, int* __restrict__ att_commit, int* __restrict__ id_commit) {
-    pdl_wait();
-    constexpr int GROUPS = SAND_BLOCK / SAND_GROUP;
-    // strides that put a warp's groups in different banks
-    __shared__ int hits[GROUPS][GROUP_HITS + 4];
-    __shared__ float terms[GROUPS][6 * GROUP_TERMS + 4];
-    const int gi = threadIdx.x / SAND_GROUP, g = threadIdx.x % SAND_GROUP;
-    const int i = blockIdx.x * GROUPS + gi;
-    if (i >= p.n) return;
-    const int lane0 = (threadIdx.x & 31) - g;
-    const unsigned mask = ((1u << SAND_GROUP) - 1u) << lane0;
-    int* hit = hits[gi];
-    float* term = terms[gi];
-    const float4 pi = tmp_in[i];
-    const float4 xi = xpre[i];
-    const float sand_coef = (SAND_COLLISION * p.mass) / (p.mass + p.mass);
-    const int c = cnt[i];
-    auto pos = [&](int e) { return e >= 0 ? tmp_in[e] : __ldg(&solid[-1 - e]); };
-    float dp = 0.0f;  // component g
-    for (int k = 0; k < c;) {
-        int m = 0;
-        for (; k < c && m <= GROUP_HITS - 4 * SAND_GROUP; k += 4 * SAND_GROUP) {
-            int e[4];
-            float4 o[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++) e[u] = nbr[(size_t)min(k + u * SAND_GROUP + g, c - 1) * p.n + i];
-#pragma unroll
-            for (int u = 0; u < 4; u++) o[u] = pos(e[u]);
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const float d2 = sdot(pi.x - o[u].x, pi.y - o[u].y, pi.z - o[u].z);
-                const bool in = k + u * SAND_GROUP + g < c && !(d2 > q.reach2);
-                const unsigned who = __ballot_sync(mask, in) >> lane0;
-                if (in) hit[m + __popc(who & ((1u << g) - 1u))] = e[u];
-                m += __popc(who);
-            }
-        }
-        __syncwarp(mask);
-        for (int t0 = 0; t0 < m; t0 += GROUP_TERMS) {
-            const int t1 = min(m - t0, GROUP_TERMS);
-            for (int j = g; j < t1; j += SAND_GROUP) {
-                const int e = hit[t0 + j];
-                const float4 pj = pos(e);
-                const bool sand_j = e >= 0;
-                const SandTerm o = sand_pair(q, sand_j, sand_j ? sand_coef : SAND_COLLISION, pi, pj, xi,
-                                             sand_j ? xpre[e] : pj);
-                term[j] = o.tx;
-                term[GROUP_TERMS + j] = o.ty;
-                term[2 * GROUP_TERMS + j] = o.tz;
-                term[3 * GROUP_TERMS + j] = o.fx;
-                term[4 * GROUP_TERMS + j] = o.fy;
-                term[5 * GROUP_TERMS + j] = o.fz;
-            }
-            __syncwarp(mask);
-            if (g < 3)
-                for (int j = 0; j < t1; j++) dp = (dp - term[g * GROUP_TERMS + j]) - term[(3 + g) * GROUP_TERMS + j];
-            __syncwarp(mask);
-        }
-    }
-    const float dpy = __shfl_sync(mask, dp, lane0 + 1), dpz = __shfl_sync(mask, dp, lane0 + 2);
-    if (g) return;
-    const float4 s = sand_clamp(p, pi.x + dp, pi.y + dpy, pi.z + dpz);
-    if (!x_commit) {
-        star_out[i] = s;
-        return;
-    }
-    x_commit[i] = s;
-    v_commit[i] = make_float4((s.x - xi.x) / p.dt, (s.y - xi.y) / p.dt, (s.z - xi.z) / p.dt, 0.0f);
-    att_commit[i] = att_in[i];
-    id_commit[i] = i;
-}
-
 // ------------------------------------------------------------------ launch --
 
 static inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
-// Largest scenes whose list build and whose substeps give each particle four
-// lanes.  Measured, us per step with one lane / four in the build / four in both:
-// 5,000 particles 52.3 / 47.3 / 43.8, 10,000 (h = 1.55) 73.9 / 63.6 / 58.0,
-// 20,011 54.4 / 49.7 / 49.6, 41,000 56.8 / 53.5 / 53.1, 81,000 65.2 / 65.8 /
-// 76.9, 80,000 (h = 1.55) 90.3 / 98.6 / 109.
+// Largest scenes whose list build gives each particle four lanes.  Measured, us a
+// step with one lane / with four: 5,000 particles 52.3 / 47.3, 10,000 (h = 1.55)
+// 73.9 / 63.6, 20,011 54.4 / 49.7, 41,000 56.8 / 53.5, 81,000 65.2 / 65.8; 96
+// contexts of 2,000 to 20,000 at once 398 / 365 (h = 1.55: 469 / 505).  (Four lanes in
+// the substeps too gave a single scene of 5,000 43.8, but the 96 contexts 541.)
 constexpr int SAND_LISTS_GROUP_MAX = 45000;
-constexpr int SAND_STEP_GROUP_MAX = 16000;
 
 void launch_sand_predict(const StepParams& p, const SandParams& q, const float4* x, float4* v, float4* xs,
                          int* att, int* key, int* rank, int* count, int* status, cudaStream_t st) {
@@ -470,12 +386,8 @@ void launch_sand_substep(const StepParams& p, const SandParams& q, const float4*
                          float4* x_commit, float4* v_commit, const int* att_in, int* att_commit,
                          int* id_commit, cudaStream_t st) {
     if (p.n <= 0) return;
-    if (p.n <= SAND_STEP_GROUP_MAX)
-        launch_k(k_sand_substep_group, blocks_for(p.n, SAND_BLOCK / SAND_GROUP), SAND_BLOCK, st, pdl_enabled(), p, q,
-                 tmp_in, star_out, xpre, nbr, cnt, solid, x_commit, v_commit, att_in, att_commit, id_commit);
-    else
-        launch_k(k_sand_substep, blocks_for(p.n, SAND_BLOCK), SAND_BLOCK, st, pdl_enabled(), p, q, tmp_in, star_out,
-                 xpre, nbr, cnt, solid, x_commit, v_commit, att_in, att_commit, id_commit);
+    launch_k(k_sand_substep, blocks_for(p.n, SAND_BLOCK), SAND_BLOCK, st, pdl_enabled(), p, q, tmp_in, star_out,
+             xpre, nbr, cnt, solid, x_commit, v_commit, att_in, att_commit, id_commit);
 }
 
 }  // namespace lgb
