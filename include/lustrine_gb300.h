@@ -521,11 +521,13 @@ LUSTRINE_API int lustrine_pbf_launches_per_step(const lustrine_pbf* s);
  * keys[0..num_positions) in [0, num_cells).  sorted_indices receives the
  * input index of the k-th smallest key (equal keys in input order) and
  * counts (num_cells + 1 ints) the state the reference leaves in its counts
- * array: the first output position of every key, then num_positions.  The
- * extra scratch is taken from a pool of the library's own in the order of
- * `stream` (a cudaStream_t, NULL for the default stream) and returned to it
- * before the call ends; the call synchronises the stream.  The pool keeps up to
- * 128 MiB a device for later calls.  LUSTRINE_ERR_ARGS if a key is out of range. */
+ * array: the first output position of every key, then num_positions.  keys may
+ * overlap sorted_indices or counts (it is read whole before either is
+ * written); those two must not overlap each other.  The extra scratch is
+ * taken from a pool of the library's own in the order of `stream` (a
+ * cudaStream_t, NULL for the default stream) and returned to it before the
+ * call ends; the call synchronises the stream.  The pool keeps up to 128 MiB
+ * a device for later calls.  LUSTRINE_ERR_ARGS if a key is out of range. */
 LUSTRINE_API int lustrine_counting_sort(int* counts, const int* keys, size_t num_positions,
                                         size_t num_cells, int* sorted_indices, void* stream);
 /* Gives the scratch that lustrine_counting_sort keeps on the current device

@@ -15,9 +15,10 @@ constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 constexpr size_t scan_block_sums_ints(size_t C) { return (C + SCAN_TILE - 1) / SCAN_TILE + 1; }
 // Scratch of the standalone counting sort: count[C], status, the scan's tile
-// sums, rank[n] (also the big cells' merge space), tmp[n].
-constexpr size_t counting_sort_scratch_ints_for(size_t n, size_t C) {
-    return C + 1 + scan_block_sums_ints(C) + 2 * n;
+// sums, rank[n] (also the big cells' merge space), tmp[n], key[n] where the
+// caller's keys are copied.
+constexpr size_t counting_sort_scratch_ints_for(size_t n, size_t C, bool copy_keys) {
+    return C + 1 + scan_block_sums_ints(C) + (copy_keys ? 3 : 2) * n;
 }
 // exclusive scan count -> start (C + 1 entries); zeroes count behind it
 void launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st);
@@ -48,9 +49,11 @@ struct CountingSortScratch {
     int* block_sums;  // scan_block_sums_size(num_cells), or the step scan's tile totals
     int* rank;        // n
     int* tmp;         // n
+    int* key;         // n, or nullptr: the caller's keys are read in place
 };
-size_t counting_sort_scratch_ints(int n, int num_cells);
-CountingSortScratch counting_sort_scratch(int* base, int n, int num_cells);
+// whether the sort works on a copy of the caller's keys
+bool counting_sort_copies_keys(const int* counts, const int* keys, size_t n, size_t num_cells, const int* sorted);
+CountingSortScratch counting_sort_scratch(int* base, int n, int num_cells, bool copy_keys);
 // start: num_cells + 1 exclusive offsets; sorted: n input indices in stable key order
 void launch_counting_sort(const int* keys, int n, int num_cells, CountingSortScratch w, int* start,
                           int* sorted, cudaStream_t st);

@@ -127,13 +127,14 @@ extern "C" int lustrine_counting_sort(int* counts, const int* keys, size_t num_p
     if (!sort_args_ok(counts, keys, num_positions, num_cells, sorted_indices)) return LUSTRINE_ERR_ARGS;
     cudaStream_t st = (cudaStream_t)stream;
     const int n = (int)num_positions, C = (int)num_cells;
-    const size_t bytes = counting_sort_scratch_ints(n, C) * sizeof(int);
+    const bool copy_keys = counting_sort_copies_keys(counts, keys, num_positions, num_cells, sorted_indices);
+    const size_t bytes = counting_sort_scratch_ints_for(num_positions, num_cells, copy_keys) * sizeof(int);
     int* scratch = nullptr;
     DeviceScratch* const kept = device_scratch(true);
     cudaError_t e = kept ? cudaMallocFromPoolAsync((void**)&scratch, bytes, kept->pool, st)
                          : cudaMallocAsync((void**)&scratch, bytes, st);
     if (e != cudaSuccess) return lgb_cuda_status(e, "cudaMallocAsync");
-    CountingSortScratch w = counting_sort_scratch(scratch, n, C);
+    CountingSortScratch w = counting_sort_scratch(scratch, n, C, copy_keys);
     int bad = 0;
     const int word = take_word(kept);
     // the histogram and the status word behind it start at zero

@@ -31,10 +31,10 @@ using namespace lgb;
 
 namespace {
 
-// the sort's scratch (count[cells] + status + scan tile sums + rank, tmp[keys])
-// at the maxima, sized by the same layout function the sort uses
+// the sort's scratch (count[cells] + status + scan tile sums + rank, tmp,
+// key[keys]) at the maxima, sized by the same layout function the sort uses
 constexpr size_t kScratchInts =
-    counting_sort_scratch_ints_for((size_t)LUSTRINE_NOALLOC_MAX_KEYS, (size_t)LUSTRINE_NOALLOC_MAX_CELLS);
+    counting_sort_scratch_ints_for((size_t)LUSTRINE_NOALLOC_MAX_KEYS, (size_t)LUSTRINE_NOALLOC_MAX_CELLS, true);
 static_assert(kScratchInts * sizeof(int) <= LUSTRINE_NOALLOC_SCRATCH_BYTES,
               "scratch array larger than the documented size");
 
@@ -69,15 +69,13 @@ extern "C" int lustrine_counting_sort_noalloc(int* counts, const int* keys, size
         return LUSTRINE_ERR_ARGS;
     if (num_positions > (size_t)LUSTRINE_NOALLOC_MAX_KEYS || num_cells > (size_t)LUSTRINE_NOALLOC_MAX_CELLS)
         return LUSTRINE_ERR_TOO_LARGE;
-    if (counting_sort_scratch_ints((int)num_positions, (int)num_cells) * sizeof(int) >
-        (size_t)LUSTRINE_NOALLOC_SCRATCH_BYTES)
-        return LUSTRINE_ERR_TOO_LARGE;
     int* scratch = nullptr;
     int rc = scratch_for_current_device(&scratch);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     const int n = (int)num_positions, C = (int)num_cells;
-    CountingSortScratch w = counting_sort_scratch(scratch, n, C);
+    CountingSortScratch w = counting_sort_scratch(
+        scratch, n, C, counting_sort_copies_keys(counts, keys, num_positions, num_cells, sorted_indices));
     // the histogram and the status word start at zero; the rest is written
     // before it is read
     cudaError_t e = cudaMemsetAsync(w.count, 0, ((size_t)C + 1) * sizeof(int), st);
