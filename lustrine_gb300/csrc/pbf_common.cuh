@@ -196,8 +196,10 @@ __device__ __forceinline__ void pdl_wait() {
 }
 
 // Launch with programmatic stream serialisation allowed (when pdl is set).
+// Returns the launch's own error (a step's launches leave it to the check after
+// the last of them).
 template <typename... KArgs, typename... Args>
-inline void launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, bool pdl,
+inline cudaError_t launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t st, bool pdl,
                      Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -209,7 +211,7 @@ inline void launch_k(void (*kernel)(KArgs...), int grid, int block, cudaStream_t
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
 // Whether the launchers of the calling thread use programmatic dependent

@@ -21,7 +21,7 @@ constexpr size_t counting_sort_scratch_ints_for(size_t n, size_t C, bool copy_ke
     return C + 1 + scan_block_sums_ints(C) + (copy_keys ? 3 : 2) * n;
 }
 // exclusive scan count -> start (C + 1 entries); zeroes count behind it
-void launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st);
+cudaError_t launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st);
 int scan_block_sums_size(int C);
 // scan of the step: tile totals, then tiles scanned independently (the
 // totals scanned by one block in between past CELL_SCAN_MAX_TILES tiles);
@@ -30,8 +30,8 @@ int scan_block_sums_size(int C);
 // null): the other totals buffer, zeroed for the next prediction.
 // scan_tiles_launches: kernels it issues.
 int cell_scan_tiles(int C);
-void launch_scan_tiles(int* count, int C, int* tile_sum, int* start, cudaStream_t st, bool counted = false,
-                       int* tile_zero = nullptr);
+cudaError_t launch_scan_tiles(int* count, int C, int* tile_sum, int* start, cudaStream_t st, bool counted = false,
+                              int* tile_zero = nullptr);
 int scan_tiles_launches(int C, bool counted = false);
 // rank doubles as merge space for cells of more than a few dozen particles
 void launch_sort_tail(const int* key, int num_cells, int* rank, const int* start, const int* tie, int n,
@@ -54,9 +54,10 @@ struct CountingSortScratch {
 // whether the sort works on a copy of the caller's keys
 bool counting_sort_copies_keys(const int* counts, const int* keys, size_t n, size_t num_cells, const int* sorted);
 CountingSortScratch counting_sort_scratch(int* base, int n, int num_cells, bool copy_keys);
-// start: num_cells + 1 exclusive offsets; sorted: n input indices in stable key order
-void launch_counting_sort(const int* keys, int n, int num_cells, CountingSortScratch w, int* start,
-                          int* sorted, cudaStream_t st);
+// start: num_cells + 1 exclusive offsets; sorted: n input indices in stable key
+// order.  Returns the first launch error (nothing is launched after it).
+cudaError_t launch_counting_sort(const int* keys, int n, int num_cells, CountingSortScratch w, int* start,
+                                 int* sorted, cudaStream_t st);
 // index scatter + stabilisation fused with the reorder of the particle state
 // (v may be nullptr: not carried; aux: an optional int per particle carried
 // into the new order, e.g. the packed cells of a hashed grid; x_out nullptr:

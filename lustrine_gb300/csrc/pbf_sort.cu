@@ -459,31 +459,40 @@ __global__ void k_scatter_key(const int* __restrict__ keys, int num_cells, const
 
 static inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
 
-void launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st) {
+// The first error of a sequence of launches, none after it made.
+#define LGB_LAUNCH(...)                                       \
+    do {                                                      \
+        const cudaError_t launch_error = launch_k(__VA_ARGS__); \
+        if (launch_error != cudaSuccess) return launch_error; \
+    } while (0)
+
+cudaError_t launch_scan(int* count, int C, int* block_sums, int* start, cudaStream_t st) {
     const int nb = blocks_for(C, SCAN_TILE);
     const bool pdl = pdl_enabled();
-    launch_k(k_scan_reduce, nb, SCAN_THREADS, st, pdl, (const int*)count, C, block_sums);
-    launch_k(k_scan_sums, 1, SUMS_THREADS, st, pdl, block_sums, nb);
-    launch_k(k_scan_down, nb, SCAN_THREADS, st, pdl, count, C, (const int*)block_sums, start);
+    LGB_LAUNCH(k_scan_reduce, nb, SCAN_THREADS, st, pdl, (const int*)count, C, block_sums);
+    LGB_LAUNCH(k_scan_sums, 1, SUMS_THREADS, st, pdl, block_sums, nb);
+    LGB_LAUNCH(k_scan_down, nb, SCAN_THREADS, st, pdl, count, C, (const int*)block_sums, start);
+    return cudaSuccess;
 }
 
 int scan_block_sums_size(int C) { return scan_block_sums_ints(C); }
 
 int cell_scan_tiles(int C) { return blocks_for(C, CELL_TILE); }
 
-void launch_scan_tiles(int* count, int C, int* tile_sum, int* start, cudaStream_t st, bool counted,
-                       int* tile_zero) {
+cudaError_t launch_scan_tiles(int* count, int C, int* tile_sum, int* start, cudaStream_t st, bool counted,
+                              int* tile_zero) {
     const bool pdl = pdl_enabled();
     const int tiles = cell_scan_tiles(C);
-    if (!counted) launch_k(k_tile_sums, tiles, CELL_SCAN_THREADS, st, pdl, (const int*)count, C, tile_sum);
+    if (!counted) LGB_LAUNCH(k_tile_sums, tiles, CELL_SCAN_THREADS, st, pdl, (const int*)count, C, tile_sum);
     if (tiles <= CELL_SCAN_MAX_TILES) {
-        launch_k(k_scan_tiles<false>, tiles, CELL_SCAN_THREADS, st, pdl, count, C, (const int*)tile_sum, start,
-                 tile_zero);
+        LGB_LAUNCH(k_scan_tiles<false>, tiles, CELL_SCAN_THREADS, st, pdl, count, C, (const int*)tile_sum, start,
+                   tile_zero);
     } else {
-        launch_k(k_scan_sums, 1, SUMS_THREADS, st, pdl, tile_sum, tiles);  // in place, exclusive
-        launch_k(k_scan_tiles<true>, tiles, CELL_SCAN_THREADS, st, pdl, count, C, (const int*)tile_sum, start,
-                 tile_zero);
+        LGB_LAUNCH(k_scan_sums, 1, SUMS_THREADS, st, pdl, tile_sum, tiles);  // in place, exclusive
+        LGB_LAUNCH(k_scan_tiles<true>, tiles, CELL_SCAN_THREADS, st, pdl, count, C, (const int*)tile_sum, start,
+                   tile_zero);
     }
+    return cudaSuccess;
 }
 
 int scan_tiles_launches(int C, bool counted) {
@@ -526,24 +535,24 @@ void launch_gather_int(const int* perm, int n, const int* src, int* dst, cudaStr
 // store: 1.25 M cells in 10.0 us, against 19.1 for reduce, scan and a
 // down-sweep one cell at a time) where the caller's counts array is 16-byte
 // aligned, which its stores need; else the down-sweep.
-void launch_counting_sort(const int* keys, int n, int num_cells, CountingSortScratch w, int* start,
-                          int* sorted, cudaStream_t st) {
+cudaError_t launch_counting_sort(const int* keys, int n, int num_cells, CountingSortScratch w, int* start,
+                                 int* sorted, cudaStream_t st) {
     if (n > 0)
-        k_key_hist<<<blocks_for(n, 256), 256, 0, st>>>(keys, n, num_cells, w.key, w.rank, w.count, w.status);
+        LGB_LAUNCH(k_key_hist, blocks_for(n, 256), 256, st, false, keys, n, num_cells, w.key, w.rank, w.count,
+                   w.status);
     const bool was = pdl_enabled();
     set_pdl(n > 0);
-    if ((reinterpret_cast<size_t>(start) & 15) == 0)
-        launch_scan_tiles(w.count, num_cells, w.block_sums, start, st, false, nullptr);
-    else
-        launch_scan(w.count, num_cells, w.block_sums, start, st);
-    if (n > 0) {
-        const int* const cell = w.key ? w.key : keys;
-        launch_k(k_scatter_key, blocks_for(n, 256), 256, st, true, cell, num_cells, (const int*)w.rank,
-                 (const int*)start, n, w.tmp);
-        launch_k(k_stabilize, blocks_for(n, STAB_THREADS), STAB_THREADS, st, true, w.tmp, w.rank, cell, num_cells,
-                 (const int*)start, (const int*)nullptr, n, sorted);
-    }
+    const cudaError_t e = (reinterpret_cast<size_t>(start) & 15) == 0
+                              ? launch_scan_tiles(w.count, num_cells, w.block_sums, start, st, false, nullptr)
+                              : launch_scan(w.count, num_cells, w.block_sums, start, st);
     set_pdl(was);
+    if (e != cudaSuccess || n <= 0) return e;
+    const int* const cell = w.key ? w.key : keys;
+    LGB_LAUNCH(k_scatter_key, blocks_for(n, 256), 256, st, true, cell, num_cells, (const int*)w.rank,
+               (const int*)start, n, w.tmp);
+    LGB_LAUNCH(k_stabilize, blocks_for(n, STAB_THREADS), STAB_THREADS, st, true, w.tmp, w.rank, cell, num_cells,
+               (const int*)start, (const int*)nullptr, n, sorted);
+    return cudaSuccess;
 }
 
 // The offsets are written between the histogram and the scatter, and the

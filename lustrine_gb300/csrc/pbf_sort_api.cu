@@ -142,9 +142,7 @@ extern "C" int lustrine_counting_sort(int* counts, const int* keys, size_t num_p
     if (e == cudaSuccess) {
         int* const device_status = w.status;
         if (word >= 0) w.status = &kept->words[word];
-        const cudaError_t before = cudaPeekAtLastError();  // an earlier call's error is not this one's
-        launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
-        if (before == cudaSuccess) e = cudaPeekAtLastError();
+        e = launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
         if (word < 0 && e == cudaSuccess)
             e = cudaMemcpyAsync(&bad, device_status, sizeof(int), cudaMemcpyDeviceToHost, st);
     }

@@ -80,10 +80,11 @@ extern "C" int lustrine_counting_sort_noalloc(int* counts, const int* keys, size
     // before it is read
     cudaError_t e = cudaMemsetAsync(w.count, 0, ((size_t)C + 1) * sizeof(int), st);
     if (e != cudaSuccess) return lgb_cuda_status(e, "cudaMemsetAsync");
-    launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
+    e = launch_counting_sort(keys, n, C, w, counts, sorted_indices, st);
     int bad = 0;
-    e = cudaMemcpyAsync(&bad, w.status, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, w.status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    const cudaError_t e1 = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = e1;
     if (e != cudaSuccess) return lgb_cuda_status(e, "counting_sort_noalloc");
     return bad ? LUSTRINE_ERR_ARGS : LUSTRINE_OK;
 }
