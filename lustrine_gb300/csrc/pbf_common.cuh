@@ -127,7 +127,7 @@ struct SandParams {
     float attract_radius, blow_radius;
     float attract_coeff, blow_coeff;
     float radius, diameter;                 // particleRadius, particleDiameter
-    float reach2;                           // largest float whose square root rounds to at most diameter
+    float reach2;                           // contact_reach2(diameter): d2 > reach2 when sqrt(d2) > diameter
     float w;                                // 1 / mass
 };
 

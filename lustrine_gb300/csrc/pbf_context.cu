@@ -12,6 +12,7 @@
 #include "lustrine_gb300.h"
 #include "pbf_context.h"
 #include "pbf_kernels.h"
+#include "sand_reach.h"
 
 using namespace lgb;
 
@@ -899,11 +900,7 @@ static SandParams sand_params(const lustrine_pbf* s) {
     q.radius = s->prm.particle_radius;
     q.diameter = c.particle_diameter;
     q.w = 1.0f / s->prm.mass;  // Simulate.cpp:185
-    // sqrt(d2) > diameter exactly when d2 > reach2 (the rounded root is monotonic)
-    q.reach2 = q.diameter * q.diameter;
-    while (std::sqrt(q.reach2) > q.diameter) q.reach2 = std::nextafter(q.reach2, 0.0f);
-    while (std::isfinite(q.reach2) && std::sqrt(std::nextafter(q.reach2, INFINITY)) <= q.diameter)
-        q.reach2 = std::nextafter(q.reach2, INFINITY);
+    q.reach2 = contact_reach2(q.diameter);
     return q;
 }
 
