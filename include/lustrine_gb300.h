@@ -437,7 +437,11 @@ enum {
 LUSTRINE_API int lustrine_pbf_profile_step(lustrine_pbf* s, float dt, double* stage_ms,
                                            int* stage_launches, int num_stages);
 /* Launch shape of the PBF iteration kernels (lambda, delta-p, XSPH) and of
- * the neighbour-list build.  block and list_block: 64, 128 or 256 threads;
+ * the neighbour-list build.  block and list_block: 64, 128 or 256 threads
+ * (a list build of 256 takes four lanes a particle on dense grids of few
+ * particles: up to 11,000 with 16-bit records, up to 20,000 with column lists
+ * but those of LUSTRINE_PRECISION_MIXED; faster for one scene on an empty
+ * GPU, slower where many contexts share it);
  * unroll: neighbour gathers in flight per thread of the lambda and delta-p
  * passes, 1, 2, 4 or 8; xsph_unroll: the same for the XSPH pass (0 in
  * lustrine_pbf_set_tuning: as unroll); particles_per_thread: 1 or 2 particles
@@ -452,8 +456,9 @@ LUSTRINE_API int lustrine_pbf_profile_step(lustrine_pbf* s, float dt, double* st
  * 65,535 in contexts of fewer than 2^24 fluid particles, wide records
  * otherwise; elsewhere the step keeps column lists whatever list_format
  * says).  Until a shape is set or autotuned, get_tuning reports the library's
- * default, and the step itself picks the gathers in flight by list format and
- * particle count (the results are the same bits in every shape). */
+ * default, and the step itself picks the gathers in flight and the list
+ * build's block by list format and particle count (the results are the same
+ * bits in every shape). */
 enum {
     LUSTRINE_LISTS_COLUMN = 0,       /* count + column-major 32-bit entries */
     LUSTRINE_LISTS_COMPACT = 1,      /* 16-byte records: count, scene's first slot, 6 (+8) 16-bit offsets */

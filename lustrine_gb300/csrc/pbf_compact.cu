@@ -12,7 +12,7 @@ void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4
                           const int* cell_sorted, const int* fstart, const float4* solid, const int* solid_cell,
                           const int* sstart, int* nbr, int* cnt, float* rho, int* status, cudaStream_t st) {
     const bool pdl = pdl_enabled();
-    if (p.n <= LISTS_GROUP_MAX_COMPACT && !p.hash_bits && !p.wide) {
+    if (B == LISTS_GROUP_BLOCK && p.n <= lists_group_max(p.hash_bits != 0, true, p.wide != 0, false)) {
         constexpr int GB = LISTS_GROUP_BLOCK;
         launch_k(p.frame ? k_lists_compact_group<GB, true> : k_lists_compact_group<GB, false>, blocks_for(p.n, GB / 4),
                  GB, st, pdl, p, cp, xs, key_sorted, cell_sorted, fstart, nbr, cnt, rho, status);
@@ -45,11 +45,6 @@ void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4
 // (ListFormatOf); the lambda pass | 4 in the scene frame
 static int compact_fcode(const StepParams& p) { return 8 | (p.wide == 2 ? 32 : (p.wide ? 16 : 0)); }
 
-// Contexts of 2^24 particles and more: the passes of 32-bit records come in
-// one shape, the best one of large scenes.
-#define LGB_ONE_SHAPE(KERNEL, FF, ...) \
-    launch_k(KERNEL<FF, 1, 256>, blocks_for(p.n, 256), 256, st, pdl_enabled(), __VA_ARGS__)
-
 void launch_lambda_compact(const Tuning& tu, const StepParams& p, float4* xs, const int* nbr, const int* cnt,
                            const float4* solid, float* rho, cudaStream_t st) {
     switch (compact_fcode(p) | (p.frame ? 4 : 0)) {
@@ -57,8 +52,8 @@ void launch_lambda_compact(const Tuning& tu, const StepParams& p, float4* xs, co
         case 12: TUNE_CASE(k_lambda, 12, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
         case 24: TUNE_CASE(k_lambda, 24, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
         case 28: TUNE_CASE(k_lambda, 28, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
-        case 40: LGB_ONE_SHAPE(k_lambda, 40, p, xs, nbr, cnt, solid, rho); break;
-        default: LGB_ONE_SHAPE(k_lambda, 44, p, xs, nbr, cnt, solid, rho); break;
+        case 40: TUNE_CASE(k_lambda, 40, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
+        default: TUNE_CASE(k_lambda, 44, tu, p.n, st, p, xs, nbr, cnt, solid, rho); break;
     }
 }
 
@@ -68,7 +63,7 @@ void launch_delta_compact(const Tuning& tu, const StepParams& p, const CellPack&
     switch (compact_fcode(p)) {
         case 8: TUNE_CASE(k_delta, 8, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
         case 24: TUNE_CASE(k_delta, 24, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
-        default: LGB_ONE_SHAPE(k_delta, 40, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
+        default: TUNE_CASE(k_delta, 40, tu, p.n, st, p, cp, xs, xs_out, nbr, cnt, solid, key_sorted, x, v_out); break;
     }
 }
 
@@ -77,11 +72,6 @@ void launch_xsph_compact(const Tuning& tx, const StepParams& p, const CellPack& 
                          float4* v_out, float4* xs_next, int* key, int* rank, int* count, int* cellk,
                          int* tile_count, cudaStream_t st) {
     const int f = compact_fcode(p);
-    if (f == 40) {
-        LGB_ONE_SHAPE(k_xsph_compact, 40, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next, key, rank,
-                      count, cellk, tile_count);
-        return;
-    }
     if (tx.unroll <= 1) {  // the 32-register kernel, one gather in flight
         const int B = tx.block <= 64 ? 64 : (tx.block <= 128 ? 128 : 256);
 #define LGB_XC(FF, BB)                                                                                  \
@@ -94,7 +84,8 @@ void launch_xsph_compact(const Tuning& tx, const StepParams& p, const CellPack& 
         else LGB_XC(FF, 256);              \
     } while (0)
         if (f == 8) LGB_XCB(8);
-        else LGB_XCB(24);
+        else if (f == 24) LGB_XCB(24);
+        else LGB_XCB(40);
 #undef LGB_XCB
 #undef LGB_XC
         return;
@@ -102,7 +93,9 @@ void launch_xsph_compact(const Tuning& tx, const StepParams& p, const CellPack& 
     switch (f) {
         case 8: TUNE_CASE(k_xsph, 8, tx, p.n, st, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next, key,
                           rank, count, cellk, tile_count); break;
-        default: TUNE_CASE(k_xsph, 24, tx, p.n, st, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next,
+        case 24: TUNE_CASE(k_xsph, 24, tx, p.n, st, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next,
+                           key, rank, count, cellk, tile_count); break;
+        default: TUNE_CASE(k_xsph, 40, tx, p.n, st, p, cp, xs, v_in, nbr, cnt, key_sorted, x_out, v_out, xs_next,
                            key, rank, count, cellk, tile_count); break;
     }
 }

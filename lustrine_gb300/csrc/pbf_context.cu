@@ -287,19 +287,26 @@ static int compact_now(const lustrine_pbf* s) {
 //     200 scenes of 3.0 M 573 / 545 with 1 and 4 (4 and 4: 576)
 //   24-bit records: 200,000 62.1 (2 and 2: 63.2), 600,000 162.5 / 161.8,
 //     2 M 497 / 492 (4 and 4: 522)
+//   32-bit records: 18 M (with a fourth of the upload) 4,183 / 3,873 with 1 and 1
+//     in blocks of 256 (4 and 4: 4,254)
 constexpr int ONE_WAVE = 152 * 9 * 128;
 constexpr int XSPH_WIDE_MAX = 250000;
 static Tuning launch_shape(const lustrine_pbf* s, int format) {
     Tuning t = s->tune;
     if (s->tune_set) return t;
-    const bool small = s->n <= ONE_WAVE;
-    if (format == LUSTRINE_LISTS_COMPACT_WIDE) {
+    const bool small = s->n <= ONE_WAVE, cells = s->mixed() && !s->sp.frame;
+    if (s->n <= lists_group_max(s->sp.hash_bits != 0, format == LUSTRINE_LISTS_COMPACT,
+                                format == LUSTRINE_LISTS_COMPACT_WIDE, cells))
+        t.list_block = LISTS_GROUP_BLOCK;
+    if (format == LUSTRINE_LISTS_COMPACT_WIDE && s->cap >= COMPACT_MAX_N) {
+        t.block = 256;
+        t.unroll = t.xsph_unroll = 1;
+    } else if (format == LUSTRINE_LISTS_COMPACT_WIDE) {
         t.xsph_unroll = s->n <= XSPH_WIDE_MAX ? 8 : 2;
     } else if (format == LUSTRINE_LISTS_COMPACT) {
         t.unroll = small ? 4 : 1;
         t.xsph_unroll = 4;
     } else {
-        const bool cells = s->mixed() && !s->sp.frame;
         t.unroll = t.xsph_unroll = cells && !small ? 2 : 4;
     }
     return t;

@@ -126,8 +126,9 @@ void launch_xsph(bool mixed, const Tuning& tu, const StepParams& p, const CellPa
                  const float4* xs, const float4* v_in, const int* nbr, const int* cnt,
                  const int* key_sorted, float4* x_out, float4* v_out, float4* xs_next, int* key,
                  int* rank, int* count, int* cellk, int* tile_count, cudaStream_t st);
-// Up to this many particles a dense grid's list build gives each four lanes (16-bit
-// records; column lists but those of per-cell mixed positions): a small scene has
+// Up to this many particles a dense grid's list build of LISTS_GROUP_BLOCK threads gives
+// each four lanes (16-bit records; column lists but those of per-cell mixed positions;
+// a tuning with a smaller list block keeps one lane): a small scene has
 // fewer warps than the GPU has schedulers, and one lane's nine rows are a chain of
 // dependent loads.  Measured,
 // us a step with one lane / with four:
@@ -145,6 +146,9 @@ void launch_xsph(bool mixed, const Tuning& tu, const StepParams& p, const CellPa
 constexpr int LISTS_GROUP_MAX_COMPACT = 11000;
 constexpr int LISTS_GROUP_MAX_COLUMN = 20000;
 constexpr int LISTS_GROUP_BLOCK = 256;
+constexpr int lists_group_max(bool hashed, bool compact, bool wide, bool cells) {
+    return hashed || wide || cells ? 0 : (compact ? LISTS_GROUP_MAX_COMPACT : LISTS_GROUP_MAX_COLUMN);
+}
 // The same passes over compact lists (p.rec set; pbf_compact.cu).  B: the
 // list build's block size; p.pad: the passes' largest chunk.
 void launch_lists_compact(int B, const StepParams& p, const CellPack& cp, float4* xs, const int* key_sorted,

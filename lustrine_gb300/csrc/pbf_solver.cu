@@ -408,7 +408,7 @@ void launch_lists_lambda(bool mixed, const Tuning& tu, const StepParams& p, cons
     if (p.rec) {  // compact lists (pbf_compact.cu)
         launch_lists_compact(B, pp, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell, sstart, nbr, cnt,
                              rho, status, st);
-    } else if (p.n <= LISTS_GROUP_MAX_COLUMN && !p.hash_bits && (!mixed || p.frame)) {
+    } else if (B == LISTS_GROUP_BLOCK && p.n <= lists_group_max(p.hash_bits != 0, false, false, mixed && !p.frame)) {
         constexpr int GB = LISTS_GROUP_BLOCK;
         launch_k(mixed ? k_lists_lambda<false, false, GB, true, 4> : k_lists_lambda<false, false, GB, false, 4>,
                  blocks_for(p.n, GB / 4), GB, st, pdl, pp, cp, xs, key_sorted, cell_sorted, fstart, solid, solid_cell,
