@@ -9,6 +9,7 @@
 #include <initializer_list>
 #include <vector>
 
+#include "launch_shape.h"
 #include "lustrine_gb300.h"
 #include "pbf_context.h"
 #include "pbf_kernels.h"
@@ -195,7 +196,17 @@ static int derive(const lustrine_pbf_params& q, int n, int ns, StepParams* sp, C
     return LUSTRINE_OK;
 }
 
+// The contexts alive on each device.
+constexpr int kMaxDevices = 64;
+static DeviceLoad g_load[kMaxDevices];
+
+static void uncount_context(lustrine_pbf* s) {
+    if (s->device < kMaxDevices) g_load[s->device].add(-1, -(long long)s->counted_n);
+    s->counted_n = -1;
+}
+
 lustrine_pbf::~lustrine_pbf() {
+    if (counted_n >= 0) uncount_context(this);
     free_buffers();
     if (fork_ev) cudaEventDestroy(fork_ev);
     if (join_ev) cudaEventDestroy(join_ev);
@@ -273,43 +284,25 @@ static int compact_now(const lustrine_pbf* s) {
     return compact_capable(s);
 }
 
-// The launch shape of a step's passes: the one that was set or autotuned, else
-// by list format and size.  More gathers in flight shorten a particle's chain of
-// dependent loads but take registers (U = 4: 56, nine blocks of 128 per SM), so
-// they pay while all particles still fit the GPU at once, ONE_WAVE of them.
-// Measured, us per step at the fixed shape (2 gathers, 8 in XSPH) and at this
-// rule's, 4 iterations:
-//   column lists, fp32 with static particles: 77,000 63.7 / 58.8, 150,000
-//     87.7 / 74.3, 262,144 99.6 / 94.8, 500,000 155 / 153
-//   column lists, per-cell mixed: 150,000 94.8 / 88.0 with 4 and 4 (2 and 2:
-//     93.7), 300,000 128 / 126 with 2 and 2 (4 and 4: 132), 3 M hashed 1141 / 1119
-//   16-bit records: 10,000 37.1 / 35.5, 37 scenes of 157,443 73.4 / 69.9;
-//     200 scenes of 3.0 M 573 / 545 with 1 and 4 (4 and 4: 576)
-//   24-bit records: 200,000 62.1 (2 and 2: 63.2), 600,000 162.5 / 161.8,
-//     2 M 497 / 492 (4 and 4: 522)
-//   32-bit records: 18 M (with a fourth of the upload) 4,183 / 3,873 with 1 and 1
-//     in blocks of 256 (4 and 4: 4,254)
-constexpr int ONE_WAVE = 152 * 9 * 128;
-constexpr int XSPH_WIDE_MAX = 250000;
-static Tuning launch_shape(const lustrine_pbf* s, int format) {
-    Tuning t = s->tune;
-    if (s->tune_set) return t;
-    const bool small = s->n <= ONE_WAVE, cells = s->mixed() && !s->sp.frame;
-    if (s->n <= lists_group_max(s->sp.hash_bits != 0, format == LUSTRINE_LISTS_COMPACT,
-                                format == LUSTRINE_LISTS_COMPACT_WIDE, cells))
-        t.list_block = LISTS_GROUP_BLOCK;
-    if (format == LUSTRINE_LISTS_COMPACT_WIDE && s->cap >= COMPACT_MAX_N) {
-        t.block = 256;
-        t.unroll = t.xsph_unroll = 1;
-    } else if (format == LUSTRINE_LISTS_COMPACT_WIDE) {
-        t.xsph_unroll = s->n <= XSPH_WIDE_MAX ? 8 : 2;
-    } else if (format == LUSTRINE_LISTS_COMPACT) {
-        t.unroll = small ? 4 : 1;
-        t.xsph_unroll = 4;
-    } else {
-        t.unroll = t.xsph_unroll = cells && !small ? 2 : 4;
+// s counted with the contexts of its device, for its present capacity.
+static int count_context(lustrine_pbf* s) {
+    if (s->counted_n < 0) {
+        CK(cudaGetDevice(&s->device));
+        CK(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, s->device));
     }
-    return t;
+    if (s->device < kMaxDevices)
+        g_load[s->device].add(s->counted_n < 0, (long long)s->cap - (s->counted_n < 0 ? 0 : s->counted_n));
+    s->counted_n = s->cap;
+    return LUSTRINE_OK;
+}
+
+// The launch shape of a step's passes: the one that was set or autotuned, else
+// the default, by the load when the step is launched or captured.
+static Tuning launch_shape(const lustrine_pbf* s, int format) {
+    if (s->tune_set) return s->tune;
+    const bool cells = s->mixed() && !s->sp.frame;
+    const bool crowd = s->device < kMaxDevices && crowded(g_load[s->device], cells, s->sms);
+    return default_shape(s->tune, format, s->n, s->cap, s->sp.hash_bits != 0, cells, crowd, s->sms);
 }
 
 // Device buffers for s->cap fluid particles (s->n of them active).
@@ -413,6 +406,7 @@ extern "C" int lustrine_pbf_create(const lustrine_pbf_params* p, int n_fluid, in
         return LUSTRINE_ERR_CUDA;
     }
     rc = ctx_alloc(s);
+    if (!rc) rc = count_context(s);
     if (rc) {
         delete s;
         return rc;
@@ -437,7 +431,8 @@ extern "C" int lustrine_pbf_reserve(lustrine_pbf* s, int capacity) {
     s->cp = cp;
     s->cap = capacity;
     s->steps_done = 0;
-    return ctx_alloc(s);
+    rc = count_context(s);
+    return rc ? rc : ctx_alloc(s);
 }
 
 // Batch geometry: every scene's grid and box, cells numbered scene after
@@ -599,6 +594,7 @@ extern "C" int lustrine_batch_create(const lustrine_pbf_params* p, int num_scene
     s->sp.scene_of = s->d_scene_of;
     s->sp.solid_scene_of = s->d_solid_scene_of;
     rc = setup_onchip(s);
+    if (!rc) rc = count_context(s);
     if (rc) {
         delete s;
         return rc;

@@ -27,6 +27,8 @@ struct lustrine_pbf {
     int n = 0, ns = 0;
     int cap = 0;  // fluid particles the buffers hold (n <= cap; sources append up to it)
     cudaStream_t stream = nullptr;
+    int device = 0, sms = 0;  // of the context's creation
+    int counted_n = -1;       // particles counted with the device's contexts; -1: not counted
 
     // fluid state, two sides: the committed state is on side `cur`; a step
     // sorts it into side 1 - cur and solves there.

@@ -137,12 +137,12 @@ void launch_xsph(bool mixed, const Tuning& tu, const StepParams& p, const CellPa
 //     10,000   33.5 / 30.8    48.7 / 44.6
 //     20,000   35.6 / 31.7    54.6 / 48.8
 //     40,000   36.1 / 35.0    52.7 / 51.1
-// Where many contexts overlap on the GPU the lanes cost instructions and blocks:
-// 512 scenes of 1,024 to 65,536 particles, a context each, take 1.68 ms a step with
-// one lane, 1.74 with four up to 11,000 particles (256 threads a block; 1.79 with
-// 128), 2.00 up to 45,000; 96 scenes of 2,000 to 20,000 on voxels 0.45 and 0.47,
-// with per-cell mixed positions (64 registers) 0.49 and 0.56 (one by one 49.6 / 46.4
-// us at 10,000), which keep one lane.
+// Up to six contexts together gain too (compact, 11,000: 65 us a step with one lane
+// / 60; four of 15,000 59 / 57, six 68 / 67, where the gain ends: hence the lines at
+// 11,000 and, on voxels, whose walks are longer, 20,000).  Where many
+// contexts overlap on the GPU the lanes cost instructions and blocks, and the default
+// shape takes one (launch_shape.h).  Per-cell mixed positions (64 registers) keep
+// one: alone 49.6 / 46.4 us at 10,000, 96 contexts 0.49 and 0.56 ms.
 constexpr int LISTS_GROUP_MAX_COMPACT = 11000;
 constexpr int LISTS_GROUP_MAX_COLUMN = 20000;
 constexpr int LISTS_GROUP_BLOCK = 256;
