@@ -166,8 +166,9 @@ __device__ __forceinline__ float dot3e(float x, float y, float z) {
 
 __device__ __forceinline__ float hdiff(const StepParams& p, float r2) { return fmaxf(__fsub_rn(p.h2, r2), 0.0f); }
 
-// The argument is never subnormal, so the flush-to-zero form of rsqrtf gives
-// the same bits without the scaling around the instruction.  CELLS (per-cell
+// The argument is never subnormal, so the flush-to-zero form of rsqrtf needs no
+// scaling around the instruction; it gives rsqrtf's bits for every float r2 >= 0
+// (all of them compared on the device).  CELLS (per-cell
 // mixed passes) keeps rsqrtf: there the shorter form leaves ptxas a schedule
 // that loses more than the instructions gain (lambda pass of 1 M hashed
 // particles 20.3 -> 22.3 us; fp32 column lists of 262,144 10.8 -> 9.2).

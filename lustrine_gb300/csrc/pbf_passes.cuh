@@ -318,7 +318,7 @@ struct DroppedEntries {
 #pragma unroll
         for (int u = 0; u < W; u++)
             if (in[u] && c++ >= p.max_nbrs)
-                lambda_accumulate<KAHAN>(p, a, rel_entry<MIXED>(p, self, load_entry(e[u], xs, solid), e[u]),
+                lambda_accumulate<KAHAN, MIXED>(p, a, rel_entry<MIXED>(p, self, load_entry(e[u], xs, solid), e[u]),
                                          entry_solid(e[u]));
     }
 };
