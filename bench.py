@@ -340,42 +340,14 @@ def cpu_sand_rate(scene, x, v, reps=3):
     return scene.n * 4 / t, t
 
 
-def run_reference(args, world, rank):
-    """The reference arm: the reference's fluid step (the oracle's restatement
-    of simulate_fluid, bit-exact with the compiled reference; one solver
-    iteration) over the same 512 scenes, scenes spread over every host core.
-    One step = every scene stepped once from its initial state (a snapshot,
-    so every step costs the same)."""
-    if rank != 0:
-        return
-    from lustrine_gb300 import scenes
-    counts = [int(c) for c in scenes.batched_counts(NUM_SCENES)]
-    cpu = CpuScenes(NUM_SCENES)
-    idx = list(range(NUM_SCENES))
-    for _ in range(args.warmup):
-        cpu.step(idx, counts)
-    walls = []
-    parts = 0
-    for _ in range(args.steps):
-        w, parts = cpu.step(idx, counts)
-        walls.append(w)
-    cpu.close()
-    wall = statistics.median(walls)
-    value = parts / wall
-    line = {
-        "impl": "reference", "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": args.gpus,
-        "steps": args.steps, "warmup": args.warmup, "ms_per_step": wall * 1e3,
-        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
-        "data": "synthetic (seeded jittered dam-break blocks, log-uniform scene sizes)",
-        "config": {"workload": WORKLOAD, "scenes": NUM_SCENES, "fluid_particles": parts,
-                   "solver_iterations": 1, "semantics": "reference simulate_fluid, one pass per step",
-                   "parallelism": f"{cpu.workers} host processes, whole scenes each"},
-        "cpu_baseline": {"value": value, "unit": UNIT, "cores": cpu.workers, "kind": "port",
-                         "sample": f"all {NUM_SCENES} scenes per step, median of {args.steps} steps, "
-                                   f"each scene from its initial state"},
-        "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
-    }
-    print(json.dumps(line), flush=True)
+def run_reference(rank):
+    """The reference arm is the reference itself or nothing: it is not
+    installed beside this repository.  (Its step restated by the oracle is the
+    own arm's cpu_baseline.)"""
+    if rank == 0:
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference is a C++/CMake program without a Python package, and its "
+                                         "sources are not in this tree"}), flush=True)
 
 
 # -------------------------------------------------------------- GPU legs --
@@ -946,7 +918,7 @@ def main():
     args = parse()
     world, rank, local = dist_setup(args)
     if args.impl == "reference":
-        run_reference(args, world, rank)
+        run_reference(rank)
     else:
         run_ours(args, world, rank, local)
     if world > 1:
