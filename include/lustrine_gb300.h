@@ -531,8 +531,11 @@ LUSTRINE_API int lustrine_pbf_launches_per_step(const lustrine_pbf* s);
  * written); those two must not overlap each other.  The extra scratch is
  * taken from a pool of the library's own in the order of `stream` (a
  * cudaStream_t, NULL for the default stream) and returned to it before the
- * call ends; the call synchronises the stream.  The pool keeps up to 128 MiB
- * a device for later calls.  LUSTRINE_ERR_ARGS if a key is out of range. */
+ * call ends; the call synchronises the stream (so it fails, and ends the
+ * capture, where its stream is captured, where its thread captures another one
+ * other than in relaxed mode, or where any thread captures in global mode).
+ * The pool keeps up to 128 MiB a device for later calls.  LUSTRINE_ERR_ARGS if
+ * a key is out of range. */
 LUSTRINE_API int lustrine_counting_sort(int* counts, const int* keys, size_t num_positions,
                                         size_t num_cells, int* sorted_indices, void* stream);
 /* Gives the scratch that lustrine_counting_sort keeps on the current device

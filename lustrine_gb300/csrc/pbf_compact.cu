@@ -1,6 +1,6 @@
 // pbf_compact.cu -- launchers of the PBF passes over compact neighbour lists
 // (16-byte records of 16-bit scene-local entries, or wide records of 24- or
-// 32-bit slots; see CompactLists and walk_compact in pbf_passes.cuh).  The
+// 32-bit slots; see COMPACT_INLINE in pbf_common.cuh and walk_compact in pbf_passes.cuh).  The
 // kernels are the templates of pbf_passes.cuh with F bit 3 (compact) and bits
 // 4 and 5 (24- and 32-bit records); this translation unit instantiates them, pbf_solver.cu
 // the column-list ones.

@@ -36,9 +36,6 @@ int scan_tiles_launches(int C, bool counted = false);
 // rank doubles as merge space for cells of more than a few dozen particles
 void launch_sort_tail(const int* key, int num_cells, int* rank, const int* start, const int* tie, int n,
                       int* tmp, int* perm, cudaStream_t st);
-void launch_gather_state(const int* perm, int n, const int* key, const float4* x, const float4* xs,
-                         const float4* v, const int* id, int* key_out, float4* x_out,
-                         float4* xs_out, float4* v_out, int* id_out, cudaStream_t st);
 void launch_gather_solid(const int* perm, int n, const float4* src, float4* dst, cudaStream_t st);
 // Standalone stable counting sort of caller keys (Sorting::counting_sort,
 // src/neighbors/Sorting.cpp:12-34): scratch carved from one 16-byte aligned int
@@ -99,8 +96,8 @@ void launch_sand_substep(const StepParams& p, const SandParams& q, const float4*
 
 // pbf_solver.cu (PBF; mixed = cell index + offset representation)
 // cellk: packed cell of every particle on a hashed grid (nullptr when dense)
-// tile_count (may be null): per-tile totals of the step's cell scan, counted
-// as the histogram is (one atomic per tile a warp touches)
+// tile_count: per-tile totals of the step's cell scan, counted as the histogram
+// is (a block sums its first particle's tile, TileSum in pbf_device.cuh)
 void launch_predict(bool mixed, const StepParams& p, const CellPack& cp, const float4* x, const float4* v,
                     float4* xs, int* key, int* rank, int* count, int* cellk, int* tile_count, cudaStream_t st);
 void launch_key(bool mixed, const StepParams& p, const CellPack& cp, const float4* pos, int m,

@@ -23,7 +23,8 @@
 // Neighbour list entry (int32, column lists): bits 0-24 slot, then the
 // neighbour's cell offset from the particle's cell, 2 bits per axis as d + 1
 // (x in 25-26, y in 27-28, z in 29-30), bit 31 set for solids.  Compact
-// lists (no cell codes, no solids): 16-byte records, see CompactLists.
+// lists (no cell codes, no solids): 16-byte records, see COMPACT_INLINE in
+// pbf_common.cuh.
 //
 // Grids: dense (cell id = offset + y gX gZ + x gZ + z; the three cells of a
 // stencil row are consecutive ids) or hashed (the counting sort runs over
@@ -97,7 +98,7 @@ __global__ void k_mark_solid_near(StepParams p, CellPack cp, const float4* __res
 }
 
 // List formats: column lists, or compact lists in one of three records
-// (CompactLists in pbf_common.cuh): 16-bit offsets from the scene's first slot,
+// (pbf_common.cuh): 16-bit offsets from the scene's first slot,
 // 24-bit slots, 32-bit slots.
 enum : int { L_COLUMN = 0, L_C16 = 1, L_C24 = 2, L_C32 = 3 };
 
@@ -319,7 +320,7 @@ struct DroppedEntries {
         for (int u = 0; u < W; u++)
             if (in[u] && c++ >= p.max_nbrs)
                 lambda_accumulate<KAHAN, MIXED>(p, a, rel_entry<MIXED>(p, self, load_entry(e[u], xs, solid), e[u]),
-                                         entry_solid(e[u]));
+                                                entry_solid(e[u]));
     }
 };
 
@@ -348,10 +349,11 @@ __device__ __forceinline__ void walk_range(const StepParams& p, const float4& se
             if (MIXED) {
                 const int cz = dz0 + (t + u >= b1) + (t + u >= b2);
                 e[u] += cz << 29;
-                d.x=__fadd_rn(d.x, axis_shift(p.cell, code, 25)); d.y=__fadd_rn(d.y, axis_shift(p.cell, code, 27));
+                d.x = __fadd_rn(d.x, axis_shift(p.cell, code, 25));
+                d.y = __fadd_rn(d.y, axis_shift(p.cell, code, 27));
                 d.z = __fadd_rn(d.z, -(float)cz * p.cell);
             }
-            in[u] = u < left && u != self_at && dot3e(d.x,d.y,d.z) <= p.h2;
+            in[u] = u < left && u != self_at && dot3e(d.x, d.y, d.z) <= p.h2;
         }
         out.take(p, e, in);
     }
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(B) k_lists_compact_group(StepParams p, CellPac
 }
 
 // Compact lists (no static particles, fp32 pair offsets).
-// Held to 12 blocks of 128 threads per SM (40 registers, a few bytes
+// Held to 12 blocks of 128 threads per SM (40 registers, at most 36 bytes
 // spilled): the extra resident warps hide more of the gathers' latency
 // (config 3: 0.382 -> 0.353 ms a step; a walk that loads the next row's
 // bounds ahead, or 4 gathers in flight, was slower).
@@ -977,9 +979,9 @@ __device__ __forceinline__ void delta_finish(const StepParams& p, const CellPack
 // With one particle per thread and up to 2 gathers in flight the kernel
 // fits 40 registers without spilling: 6 blocks of 256 threads per SM instead
 // of 5 (a 262,144-particle pass then takes 1.12 waves of the GPU instead of
-// 1.35).  Compact lists with one gather in flight fit 32 registers without
-// spilling (their steps have an integer s_corr exponent: no powf): 16 blocks
-// of 128 threads per SM, the whole SM's warps.  P = 2:
+// 1.35).  Compact lists with one gather in flight fit 32 registers with at
+// most 20 bytes spilled (their steps have an integer s_corr exponent: no powf):
+// 16 blocks of 128 threads per SM, the whole SM's warps.  P = 2:
 // two particles per thread (B apart), their lists walked together.
 template <int F, int U, int B, int P = 1>
 __global__ void __launch_bounds__(B, ((F & 8) && U == 1) ? 2048 / B : ((U <= 2 && P == 1) ? 1536 / B : 1))
@@ -1162,10 +1164,11 @@ __global__ void __launch_bounds__(B) k_xsph(StepParams p, CellPack cp, const flo
                       tile_count);
 }
 
-// Compact lists (F = 8, 24) with one gather in flight: registers capped at 32
-// for every warp slot of the SM (at most 16 bytes spilled; config 3 XSPH 0.175 ->
-// 0.141 ms at step 5, 0.239 -> 0.219 ms at step 100 against the best
-// uncapped shape).  More gathers in flight keep k_xsph.
+// Compact lists (F = 8, 24, 40) with one gather in flight: registers capped at 32
+// for every warp slot of the SM (8 bytes spilled with 16-bit records, 88 with
+// 24-bit ones, none with 32-bit ones; config 3 XSPH 0.175 -> 0.141 ms at step 5,
+// 0.239 -> 0.219 ms at step 100 against the best uncapped shape).  More
+// gathers in flight keep k_xsph.
 template <int F, int U, int B>
 __global__ void __launch_bounds__(B, 2048 / B) k_xsph_compact(
     StepParams p, CellPack cp, const float4* __restrict__ xs, const float4* __restrict__ v_in,
@@ -1239,7 +1242,8 @@ static inline int blocks_for(int n, int t) { return (n + t - 1) / t; }
     } while (0)
 // fcode: bit 0 mixed (cell-relative pair offsets), bit 1 static particles,
 // bit 2 (the lambda pass only) the scene frame's compensated sums, bit 3
-// compact lists (with bit 2 at most), bit 4 their wide records
+// compact lists (with bit 2 at most), bit 4 their 24-bit and bit 5 their 32-bit
+// records
 #define TUNE_DISPATCH(KERNEL, fcode, tu, N, ST, ...)                                            \
     do {                                                                                        \
         switch (fcode) {                                                                        \
